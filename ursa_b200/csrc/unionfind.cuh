@@ -16,6 +16,17 @@ __device__ __forceinline__ uint32_t uf_parent(const uint32_t* p, uint32_t x) {
   return *(const volatile uint32_t*)&p[x];
 }
 
+// The same read through L1 (global memory only).  A cached parent may be
+// stale, which costs steps and no correctness: what was once an ancestor of x
+// stays one, parents stay smaller than their children, and a stale root is
+// found out by the compare-and-swap that hooks it.  Reads past L1 all meet at
+// the L2 slice that holds the largest tree's root.
+__device__ __forceinline__ uint32_t uf_parent_l1(const uint32_t* p, uint32_t x) {
+  uint32_t v;
+  asm volatile("ld.global.ca.u32 %0, [%1];" : "=r"(v) : "l"(p + x) : "memory");
+  return v;
+}
+
 // Root of x with intermediate pointer jumping (parent[x] < x off the root).
 __device__ __forceinline__ uint32_t uf_find(uint32_t* p, uint32_t x) {
   uint32_t par = uf_parent(p, x);
@@ -30,8 +41,29 @@ __device__ __forceinline__ uint32_t uf_find(uint32_t* p, uint32_t x) {
   return par;
 }
 
+// The same through L1 for the first kUfShort links (past them a walk wants
+// the jumps that others have stored), and x's own parent stored at the end.
+constexpr int kUfShort = 4;
+__device__ __forceinline__ uint32_t uf_find_l1(uint32_t* p, uint32_t x) {
+  uint32_t par = uf_parent_l1(p, x);
+  if (par != x) {
+    uint32_t prev = x, next;
+    int links = 0;
+    while (par > (next = links < kUfShort ? uf_parent_l1(p, par) : uf_parent(p, par))) {
+      links++;
+      p[prev] = next;
+      prev = par;
+      par = next;
+    }
+    if (links > 1) p[x] = par;
+  }
+  return par;
+}
+
+template <bool kL1 = false>
 __device__ __forceinline__ void uf_unite(uint32_t* p, uint32_t a, uint32_t b) {
-  uint32_t ra = uf_find(p, a), rb = uf_find(p, b);
+  uint32_t ra = kL1 ? uf_find_l1(p, a) : uf_find(p, a);
+  uint32_t rb = kL1 ? uf_find_l1(p, b) : uf_find(p, b);
   // bounded by the depth of the forest; each failed CAS moves one link up
   while (ra != rb) {
     if (ra < rb) {
