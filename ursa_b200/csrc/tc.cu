@@ -54,9 +54,29 @@ __device__ __forceinline__ uint32_t tc_hash(uint32_t w, uint32_t bits) {
   return (w * 0x9E3779B1u) >> (32 - bits);
 }
 
-constexpr uint64_t kTcWork = 16384;  // probes per work item of a warp (one suffix may exceed it)
-constexpr uint32_t kTcWarpMax = 256;  // larger N+(v): a block of kTcBlockWarps warps per item
+// N+(v) of up to kTcSearchMax elements is searched where it lies, a lane per
+// probe whatever its v; up to kTcWarpMax a warp's hash table; larger ones a
+// block's.  Most vertices have short lists and few probes: a table for each
+// of them was all latency (a chunk of 1,024 probes could take 300 tables).
+constexpr uint32_t kTcSearchMax = 24;  // five halvings
+constexpr uint32_t kTcWarpMax = 256;
 constexpr uint32_t kTcBlockWarps = 8;
+constexpr uint32_t kTcMidSlots = 2048;  // a block's table in shared memory
+
+// The vertices that take a table are listed per kind (warp, block), and the
+// probes of a list's vertices, back to back, are cut into chunks of equal
+// size (an entry's probes stay together) whatever vertices they span: a
+// vertex's in-list is cut where it is long, and the next table starts where
+// the last one ended.  At most kTcChunks chunks, so that the last ones end
+// together on a large graph; at least kTcMinWork units of kTcUnit probes
+// each.  (Pieces of up to 16K probes of one in-list, sixteen to a grab, left
+// R-MAT-16's 7,000 warps waiting for the few that drew the hubs; one cut over
+// all vertices left them skipping thousands of other kinds' lists.)
+constexpr uint32_t kTcChunks[2] = {1u << 17, 1u << 13};
+constexpr uint64_t kTcUnit = 256;
+constexpr uint64_t kTcMinWork[2] = {4, 32};
+constexpr uint32_t kTcSearchEntries = 256;  // most in-list entries per grab of a searching warp
+constexpr int kTcKinds = 2;                 // warp tables, block tables
 
 // One middle vertex v (original id) at a time: N+(v) = rank ids tgt[ob, oe)
 // (all ranked above v, ascending) in a hash table T/C of 2^bits slots (load
@@ -78,17 +98,26 @@ __device__ __forceinline__ void tc_table_fill(uint32_t* T, uint32_t bits, uint32
 }
 
 // Slot of w in the table (buckets of four keys, one 16-byte load each), or
-// kTcEmpty if absent.
+// kTcEmpty if absent or w is kTcEmpty.  The warp takes every step together
+// until its last lane is done, so that it is converged for the ballot that
+// follows.
 __device__ __forceinline__ uint32_t tc_find(const uint32_t* T, uint32_t bits, uint32_t w) {
   const uint32_t bmask = (1u << (bits - 2)) - 1u;
-  for (uint32_t b = tc_hash(w, bits - 2);; b = (b + 1) & bmask) {
+  uint32_t b = tc_hash(w, bits - 2), h = kTcEmpty;
+  bool open = w != kTcEmpty;
+  do {
     const uint4 q = *reinterpret_cast<const uint4*>(T + 4 * b);
-    if (q.x == w) return 4 * b;
-    if (q.y == w) return 4 * b + 1;
-    if (q.z == w) return 4 * b + 2;
-    if (q.w == w) return 4 * b + 3;
-    if (q.w == kTcEmpty) return kTcEmpty;  // slots fill in order: a bucket with room ends the chain
-  }
+    if (open) {
+      if (q.x == w) h = 4 * b;
+      if (q.y == w) h = 4 * b + 1;
+      if (q.z == w) h = 4 * b + 2;
+      if (q.w == w) h = 4 * b + 3;
+      // slots fill in order: a bucket with room ends the chain
+      open = h == kTcEmpty && q.w != kTcEmpty;
+    }
+    b = (b + 1) & bmask;
+  } while (__any_sync(0xffffffffu, open));
+  return h;
 }
 
 // Credits the counts kept beside the table to their w and empties it.
@@ -108,63 +137,118 @@ __device__ __forceinline__ void tc_table_flush(uint32_t* T, uint32_t* C, uint32_
   }
 }
 
-// One warp: the entries [i0, i0 + 32) of [.., ie), 32 pairs at a time with
-// stride `stride`; credits each u and returns the warp's hit count (all lanes).
-__device__ __forceinline__ uint32_t tc_pairs(uint32_t* T, uint32_t* C, uint32_t* P, uint32_t bits,
-                                             uint32_t i0, uint32_t ie, uint32_t stride,
+// Streams up to 32 (u, v) pairs' suffixes back to back through a warp: lane l
+// takes probe pb + l of the concatenation; hit(j, w) is called by every lane
+// with the pair's lane j and the element (kTcEmpty without a probe) and says
+// whether it closes a triangle.  Lane k holds pair k: the first slot b and the
+// length len of its suffix (0: no pair).  The pairs with probes are first
+// moved to the front, so that each owns at least one probe and a round finds
+// its pairs with one ballot and one OR of the ends inside the round, in place
+// of a five-step shuffle search; and each lane counts the hits of the pair
+// that moved to it from the ballot of the round's hits, in place of a
+// shared-memory atomic per hit.  Returns that count, and the lane the pair
+// came from in *from_lane.
+template <class F>
+__device__ __forceinline__ uint32_t tc_stream(uint32_t* pack, uint32_t b, uint32_t len,
+                                              const uint32_t* __restrict__ tgt,
+                                              uint32_t* from_lane, F&& hit) {
+  const uint32_t FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const uint32_t lt = (1u << lane) - 1u;
+  const uint32_t some = __ballot_sync(FULL, len != 0);
+  const int count = __popc(some);
+  if (len) pack[__popc(some & lt)] = lane;
+  __syncwarp();
+  const uint32_t from = lane < count ? pack[lane] : 0u;
+  __syncwarp();
+  *from_lane = from;
+  b = __shfl_sync(FULL, b, from);
+  len = __shfl_sync(FULL, len, from);
+  if (lane >= count) len = 0;
+  uint32_t incl = len;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(FULL, incl, o);
+    if (lane >= o) incl += t;
+  }
+  const uint32_t total = __shfl_sync(FULL, incl, 31);
+  const uint32_t excl = incl - len;
+  const uint32_t start = b - excl;  // probe p of pair k is tgt[start_k + p]
+  uint32_t c = 0;
+  for (uint32_t pb = 0; pb < total; pb += 32) {
+    // pairs that end at or before pb, and those that end inside the round:
+    // one that ends after `at` probes leaves the lanes from `at` to the next
+    const uint32_t first = __popc(__ballot_sync(FULL, lane < count && incl <= pb));
+    const uint32_t at = incl - pb;
+    const bool inside = lane < count && incl > pb && at < 32;
+    const uint32_t ends = __reduce_or_sync(FULL, inside ? 1u << (at & 31) : 0u);
+    const uint32_t k = first + __popc(ends & (lt | (1u << lane)));
+    const uint32_t sk = __shfl_sync(FULL, start, k & 31);
+    const uint32_t j = __shfl_sync(FULL, from, k & 31);
+    const uint32_t p = pb + lane;
+    const bool h = hit(j, p < total ? tgt[sk + p] : kTcEmpty);
+    __syncwarp();
+    const uint32_t hits = __ballot_sync(FULL, h);
+    if (len && incl > pb && excl < pb + 32) {  // this lane's pair is in the round
+      const uint32_t lo = excl > pb ? excl - pb : 0u;
+      const uint32_t upto = at < 32 ? (1u << at) - 1u : FULL;
+      c += __popc(hits & upto & ~((1u << lo) - 1u));
+    }
+  }
+  return c;
+}
+
+// One warp: `group` (at most 32) entries of [i0, ie) at a time, `stride`
+// apart; credits each u and returns the warp's hit count (all lanes).
+__device__ __forceinline__ uint32_t tc_pairs(uint32_t* T, uint32_t* C, uint32_t* pack, uint32_t bits,
+                                             uint32_t i0, uint32_t ie, uint32_t group, uint32_t stride,
                                              const uint32_t* __restrict__ off,
                                              const uint32_t* __restrict__ tgt,
                                              const uint32_t* __restrict__ in_src,
                                              const uint32_t* __restrict__ in_pos,
                                              uint32_t* __restrict__ tri) {
   const uint32_t FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
+  const uint32_t lane = threadIdx.x & 31;
   uint32_t cv = 0;  // per lane; summed at the end
   for (; i0 < ie; i0 += stride) {
-    // 32 (u, v) pairs, one per lane: u and the part of N+(u) above v
+    // (u, v) pairs, one per lane: u and the part of N+(u) above v
     uint32_t u = 0, b = 0, len = 0;
-    if (i0 + lane < ie) {
+    if (lane < group && i0 + lane < ie) {
       u = in_src[i0 + lane];
       b = in_pos[i0 + lane] + 1;
       len = off[u + 1] - b;
     }
-    uint32_t incl = len;  // inclusive scan of the suffix lengths
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t t = __shfl_up_sync(FULL, incl, o);
-      if (lane >= o) incl += t;
-    }
-    const uint32_t total = __shfl_sync(FULL, incl, 31);
-    const uint32_t start = b - (incl - len);  // element p of pair j is tgt[start_j + p]
-    // the suffixes streamed back to back, lane l on element pb + l of pair
-    // j (the first pair whose inclusive end exceeds it: a shuffle binary
-    // search, since one round can span many short suffixes)
-    for (uint32_t pb = 0; pb < total; pb += 32) {
-      const uint32_t p = pb + lane;
-      uint32_t j = 0;
-#pragma unroll
-      for (int step = 16; step >= 1; step >>= 1) {
-        const uint32_t t = __shfl_sync(FULL, incl, j + step - 1);
-        if (t <= p) j += step;
-      }
-      const uint32_t sj = __shfl_sync(FULL, start, j & 31);
-      if (p < total) {
-        const uint32_t h = tc_find(T, bits, tgt[sj + p]);
-        if (h != kTcEmpty) {
-          atomicAdd(&C[h], 1u);
-          atomicAdd(&P[j], 1u);
-        }
-      }
-    }
-    __syncwarp();
-    const uint32_t c = P[lane];
-    P[lane] = 0;
+    uint32_t from;
+    const uint32_t c = tc_stream(pack, b, len, tgt, &from, [&](uint32_t, uint32_t w) {
+      const uint32_t h = tc_find(T, bits, w);
+      if (h != kTcEmpty) atomicAdd(&C[h], 1u);
+      return h != kTcEmpty;
+    });
+    u = __shfl_sync(FULL, u, from);
     if (c) atomicAdd(&tri[u], c);
     cv += c;
-    __syncwarp();
   }
   return __reduce_add_sync(FULL, cv);
 }
+
+// One kind's vertices, in no order: ranks, and the work (in units) of the
+// ones before; its chunks: index of the vertex and in-list entry where each
+// starts (one past the last closes the list).
+struct TcList {
+  uint32_t* rank;
+  uint64_t* at;
+  uint32_t* chunk_i;
+  uint32_t* chunk_e;
+};
+// Device words of a call: per kind, vertices << 38 | work units of the list
+// (so at most 2^26 vertices with more than 32 of below 2^31 edges, and 2^46
+// probes), chunks in use, and the grab counters.
+constexpr int kTcWorkBits = 38;
+struct TcCtl {
+  unsigned long long size[kTcKinds];
+  unsigned long long next[kTcKinds + 1];
+  uint32_t chunks[kTcKinds];
+};
 
 struct TcArgs {
   const uint32_t* off;        // oriented CSR rows by original id
@@ -172,104 +256,189 @@ struct TcArgs {
   const uint32_t* in_off;     // in-lists of the oriented graph, by rank
   const uint32_t* in_src;     // ... holding original ids
   const uint32_t* in_pos;     // ... and the entry's slot in its row of tgt
+  const uint32_t* in_rank;    // ... and the rank of the list
   const uint32_t* vertex_of;  // rank -> original id
-  const uint32_t* item_rank;   // work items, by rank ascending: middle vertex rank
-  const uint32_t* item_begin;  // ... and their in-list entries [begin, end)
-  const uint32_t* item_end;
-  uint32_t n_items;
+  uint64_t entries;           // in-list entries of all ranks
+  uint32_t grab;              // ... taken at a time by a searching warp
+  TcList list;                // this launch's kind
+  int kind;
+  TcCtl* ctl;
   uint32_t* tri;
-  unsigned long long* next;   // item grab counter (from the end: hubs first)
-  uint32_t lo, hi;            // this launch handles |N+(v)| in (lo, hi]
 };
 
-__device__ __forceinline__ bool tc_item(const TcArgs& a, uint32_t q, uint32_t& v, uint32_t& ob,
-                                        uint32_t& oe, uint32_t& ib, uint32_t& ie,
-                                        uint32_t& bits) {
-  const uint32_t r = a.item_rank[q];
-  v = a.vertex_of[r];
-  ob = a.off[v];
-  oe = a.off[v + 1];
-  const uint32_t dv = oe - ob;
-  if (dv <= a.lo || dv > a.hi) return false;
-  ib = a.item_begin[q];
-  ie = a.item_end[q];
-  bits = 3;  // at least two buckets of four slots
-  while ((1u << bits) < 2 * dv) bits++;
-  return true;
+// A list's vertices i .. i + 31 (a lane each) between chunk starts (i0, e0)
+// and (i1, e1): vertex, N+(v) and the in-list entries to walk (ib < ie).
+struct TcRank {
+  uint32_t v, ob, dv, ib, ie;
+};
+__device__ __forceinline__ TcRank tc_rank(const TcArgs& a, uint32_t i, uint32_t count, uint32_t i0,
+                                          uint32_t e0, uint32_t i1, uint32_t e1) {
+  TcRank x{0, 0, 0, 0, 0};
+  if (i < count && i <= i1) {
+    const uint32_t r = a.list.rank[i];
+    x.v = a.vertex_of[r];
+    x.ob = a.off[x.v];
+    x.dv = a.off[x.v + 1] - x.ob;
+    x.ib = i == i0 ? e0 : a.in_off[r];
+    x.ie = i == i1 ? e1 : a.in_off[r + 1];
+  }
+  return x;
 }
 
-// Items whose middle vertex has lo < |N+(v)| <= hi = kSlots / 2: one warp per
-// item, a table per warp in shared memory (kWarps warps per block).
+// log2 of the table's slots: load <= 1/2, at least two buckets of four slots.
+__device__ __forceinline__ uint32_t tc_bits(uint32_t dv) {
+  return max(3u, 32u - (uint32_t)__clz(2 * dv - 1));
+}
+
+// Middle vertices with |N+(v)| <= kTcSearchMax: a warp takes 32 entries at a
+// time whatever their v; each probe is searched in N+(v) by bisection.
+__global__ void __launch_bounds__(256) tc_middle_search_k(TcArgs a) {
+  __shared__ uint32_t pack[8][32];
+  const uint32_t FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  while (true) {
+    unsigned long long g = 0;
+    if (lane == 0) g = atomicAdd(&a.ctl->next[kTcKinds], (unsigned long long)a.grab);
+    g = __shfl_sync(FULL, g, 0);
+    if (g >= a.entries) break;
+    const uint32_t e1 = (uint32_t)min(a.entries, (uint64_t)g + a.grab);
+    for (uint32_t e = (uint32_t)g; e < e1; e += 32) {
+      uint32_t u = 0, b = 0, len = 0, v = 0, ob = 0, dv = 0;
+      if (e + lane < e1) {
+        v = a.vertex_of[a.in_rank[e + lane]];
+        ob = a.off[v];
+        dv = a.off[v + 1] - ob;
+        if (dv != 0 && dv <= kTcSearchMax) {
+          u = a.in_src[e + lane];
+          b = a.in_pos[e + lane] + 1;
+          len = a.off[u + 1] - b;
+        }
+      }
+      if (!__any_sync(FULL, len != 0)) continue;
+      uint32_t from;
+      const uint32_t c = tc_stream(pack[wid], b, len, a.tgt, &from, [&](uint32_t j, uint32_t w) {
+        uint32_t lo = __shfl_sync(FULL, ob, j);
+        uint32_t left = __shfl_sync(FULL, dv, j);
+        if (w == kTcEmpty) left = 0;
+#pragma unroll
+        for (int step = 0; step < 5; step++) {  // the last element <= w, or the first one
+          const uint32_t half = left >> 1;
+          if (half && a.tgt[lo + half] <= w) lo += half;
+          left -= half;
+        }
+        const bool h = left && a.tgt[lo] == w;
+        if (h) atomicAdd(&a.tri[a.vertex_of[w]], 1u);
+        return h;
+      });
+      u = __shfl_sync(FULL, u, from);
+      v = __shfl_sync(FULL, v, from);
+      if (c) {
+        atomicAdd(&a.tri[u], c);
+        atomicAdd(&a.tri[v], c);
+      }
+    }
+  }
+}
+
+// Middle vertices with |N+(v)| <= kSlots / 2: a warp per chunk, a table per
+// warp in shared memory (kWarps warps per block).
 template <int kSlots, int kWarps>
 __global__ void __launch_bounds__(kWarps * 32) tc_middle_warp_k(TcArgs a) {
   extern __shared__ uint32_t tc_sm[];
+  const uint32_t FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   uint32_t* T = tc_sm + (size_t)wid * 2 * kSlots;
   uint32_t* C = T + kSlots;
-  uint32_t* P = tc_sm + (size_t)kWarps * 2 * kSlots + wid * 32;
+  uint32_t* pack = tc_sm + (size_t)kWarps * 2 * kSlots + wid * 32;
   for (int i = lane; i < kSlots; i += 32) {
     T[i] = kTcEmpty;
     C[i] = 0;
   }
-  P[lane] = 0;
   __syncwarp();
+  const uint32_t n_chunks = a.ctl->chunks[a.kind];
+  const uint32_t count = (uint32_t)(a.ctl->size[a.kind] >> kTcWorkBits);
   while (true) {
     unsigned long long g = 0;
-    if (lane == 0) g = atomicAdd(a.next, (unsigned long long)kTcGrab);
-    g = __shfl_sync(0xffffffffu, g, 0);
-    if (g >= a.n_items) break;
-    const uint64_t g_end = g + kTcGrab < a.n_items ? g + kTcGrab : a.n_items;
-    for (uint64_t q = g; q < g_end; q++) {
-      uint32_t v, ob, oe, ib, ie, bits;
-      if (!tc_item(a, (uint32_t)(a.n_items - 1 - q), v, ob, oe, ib, ie, bits)) continue;
-      tc_table_fill(T, bits, ob, oe, a.tgt, lane, 32);
-      __syncwarp();
-      const uint32_t cv = tc_pairs(T, C, P, bits, ib, ie, 32, a.off, a.tgt, a.in_src, a.in_pos, a.tri);
-      __syncwarp();
-      tc_table_flush(T, C, bits, a.vertex_of, a.tri, lane, 32);
-      if (cv && lane == 0) atomicAdd(&a.tri[v], cv);
-      __syncwarp();
+    if (lane == 0) g = atomicAdd(&a.ctl->next[a.kind], 1ull);
+    g = __shfl_sync(FULL, g, 0);
+    if (g >= n_chunks) break;
+    const uint32_t i0 = a.list.chunk_i[g], e0 = a.list.chunk_e[g];
+    const uint32_t i1 = a.list.chunk_i[g + 1], e1 = a.list.chunk_e[g + 1];
+    for (uint32_t i = i0; i < count && i <= i1; i += 32) {
+      const TcRank x = tc_rank(a, i + lane, count, i0, e0, i1, e1);
+      for (unsigned todo = __ballot_sync(FULL, x.ib < x.ie); todo; todo &= todo - 1) {
+        const int l = __ffs(todo) - 1;
+        const uint32_t v = __shfl_sync(FULL, x.v, l), ob = __shfl_sync(FULL, x.ob, l);
+        const uint32_t dv = __shfl_sync(FULL, x.dv, l);
+        const uint32_t ib = __shfl_sync(FULL, x.ib, l), ie = __shfl_sync(FULL, x.ie, l);
+        const uint32_t bits = tc_bits(dv);
+        tc_table_fill(T, bits, ob, ob + dv, a.tgt, lane, 32);
+        __syncwarp();
+        const uint32_t cv = tc_pairs(T, C, pack, bits, ib, ie, 32, 32, a.off, a.tgt, a.in_src, a.in_pos, a.tri);
+        __syncwarp();
+        tc_table_flush(T, C, bits, a.vertex_of, a.tri, lane, 32);
+        if (cv && lane == 0) atomicAdd(&a.tri[v], cv);
+        __syncwarp();
+      }
     }
   }
 }
 
-// Items whose middle vertex has |N+(v)| > lo (and <= hi): one block of
-// kWarps warps per item sharing one table -- in shared memory of `slots`
-// slots when `table` is null, else table[block * 2 * slots, +2 * slots) in
-// global memory (keys, then counts; all empty on entry, left empty).
+// The larger ones: one block of kWarps warps per chunk, sharing one table:
+// kTcMidSlots slots in shared memory up to half as many elements, else
+// table[block * 2 * slots, +2 * slots) in global memory (keys, then counts;
+// all empty on entry, left empty).  Every warp reads the vertices by itself:
+// the same values, so the same loop.
 template <int kWarps>
 __global__ void __launch_bounds__(kWarps * 32) tc_middle_block_k(TcArgs a, uint32_t* table,
                                                                  uint32_t slots) {
   extern __shared__ uint32_t tc_sm[];
-  __shared__ uint32_t pair_cnt[kWarps][32];
+  __shared__ uint32_t pack[kWarps][32];
   __shared__ unsigned long long s_g;
+  const uint32_t FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  uint32_t* T = table ? table + (size_t)blockIdx.x * 2 * slots : tc_sm;
-  uint32_t* C = T + slots;
-  uint32_t* P = pair_cnt[wid];
-  if (!table)
-    for (uint32_t i = threadIdx.x; i < slots; i += blockDim.x) {
-      T[i] = kTcEmpty;
-      C[i] = 0;
-    }
-  P[lane] = 0;
+  for (uint32_t i = threadIdx.x; i < kTcMidSlots; i += blockDim.x) {
+    tc_sm[i] = kTcEmpty;
+    tc_sm[kTcMidSlots + i] = 0;
+  }
   __syncthreads();
+  const uint32_t n_chunks = a.ctl->chunks[a.kind];
+  const uint32_t count = (uint32_t)(a.ctl->size[a.kind] >> kTcWorkBits);
   while (true) {
-    if (threadIdx.x == 0) s_g = atomicAdd(a.next, 1ull);
+    if (threadIdx.x == 0) s_g = atomicAdd(&a.ctl->next[a.kind], 1ull);
     __syncthreads();
     const unsigned long long g = s_g;
-    __syncthreads();  // read by all before thread 0 takes the next item
-    if (g >= a.n_items) break;
-    uint32_t v, ob, oe, ib, ie, bits;
-    if (!tc_item(a, (uint32_t)(a.n_items - 1 - g), v, ob, oe, ib, ie, bits)) continue;
-    tc_table_fill(T, bits, ob, oe, a.tgt, threadIdx.x, blockDim.x);
-    __syncthreads();
-    const uint32_t cv = tc_pairs(T, C, P, bits, ib + 32u * wid, ie, 32u * kWarps, a.off, a.tgt,
-                                 a.in_src, a.in_pos, a.tri);
-    if (cv && lane == 0) atomicAdd(&a.tri[v], cv);
-    __syncthreads();
-    tc_table_flush(T, C, bits, a.vertex_of, a.tri, threadIdx.x, blockDim.x);
-    __syncthreads();
+    __syncthreads();  // read by all before thread 0 takes the next chunk
+    if (g >= n_chunks) break;
+    const uint32_t i0 = a.list.chunk_i[g], e0 = a.list.chunk_e[g];
+    const uint32_t i1 = a.list.chunk_i[g + 1], e1 = a.list.chunk_e[g + 1];
+    for (uint32_t i = i0; i < count && i <= i1; i += 32) {
+      const TcRank x = tc_rank(a, i + lane, count, i0, e0, i1, e1);
+      for (unsigned todo = __ballot_sync(FULL, x.ib < x.ie); todo; todo &= todo - 1) {
+        const int l = __ffs(todo) - 1;
+        const uint32_t v = __shfl_sync(FULL, x.v, l), ob = __shfl_sync(FULL, x.ob, l);
+        const uint32_t dv = __shfl_sync(FULL, x.dv, l);
+        const uint32_t ib = __shfl_sync(FULL, x.ib, l), ie = __shfl_sync(FULL, x.ie, l);
+        const uint32_t bits = tc_bits(dv);
+        uint32_t* T = tc_sm;
+        uint32_t* C = tc_sm + kTcMidSlots;
+        if (dv > kTcMidSlots / 2) {
+          T = table + (size_t)blockIdx.x * 2 * slots;
+          C = T + slots;
+        }
+        tc_table_fill(T, bits, ob, ob + dv, a.tgt, threadIdx.x, blockDim.x);
+        __syncthreads();
+        // the entries spread over all warps: suffixes are long here, so a
+        // few tens of entries can be all the work
+        const uint32_t group = min(32u, (ie - ib + kWarps - 1) / kWarps);
+        const uint32_t cv = tc_pairs(T, C, pack[wid], bits, ib + group * wid, ie, group,
+                                     group * kWarps, a.off, a.tgt, a.in_src, a.in_pos, a.tri);
+        if (cv && lane == 0) atomicAdd(&a.tri[v], cv);
+        __syncthreads();
+        tc_table_flush(T, C, bits, a.vertex_of, a.tri, threadIdx.x, blockDim.x);
+        __syncthreads();
+      }
+    }
   }
 }
 
@@ -454,58 +623,89 @@ __global__ void entry_work_k(const uint32_t* __restrict__ off, const uint32_t* _
                              uint64_t* __restrict__ work) {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
        i += (uint64_t)gridDim.x * blockDim.x)
-    work[i] = off[in_src[i] + 1] - in_pos[i] - 1;
+    work[i] = off[in_src[i] + 1] - in_pos[i];  // and one for the entry itself
 }
 
-// Work items per rank: its in-list cut into pieces of about kTcWork probes
-// (none when N+(v) is empty or the list has no probes: v is the middle of
-// no triangle).  wp = exclusive prefix of the entries' probes.
-__global__ void item_count_k(const uint32_t* __restrict__ in_off, const uint32_t* __restrict__ off,
-                             const uint32_t* __restrict__ vertex_of,
-                             const uint64_t* __restrict__ wp, uint64_t n,
-                             uint32_t* __restrict__ cnt) {
-  for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n;
-       r += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t v = vertex_of[r];
-    const uint32_t dv = off[v + 1] - off[v];
-    const uint64_t unit = dv > kTcWarpMax ? kTcWork * kTcBlockWarps : kTcWork;
-    const uint64_t tot = wp[in_off[r + 1]] - wp[in_off[r]];
-    cnt[r] = dv ? (uint32_t)((tot + unit - 1) / unit) : 0u;
+// The ranks that take a table, listed per kind with their work (probes in
+// units, and one for the table itself).  One atomic per warp and kind gives
+// the vertices' places and the work before them together.
+__global__ void tc_lists_k(const uint32_t* __restrict__ in_off, const uint32_t* __restrict__ off,
+                           const uint32_t* __restrict__ vertex_of, const uint64_t* __restrict__ wp,
+                           uint64_t n, TcList warp_list, TcList block_list, TcCtl* ctl) {
+  const uint32_t FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t r0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~31ull; r0 < n; r0 += stride) {
+    const uint64_t r = r0 + lane;
+    int kind = -1;
+    unsigned long long x = 0;
+    if (r < n) {
+      const uint32_t b = in_off[r], e = in_off[r + 1];
+      if (b != e) {
+        const uint32_t v = vertex_of[r];
+        const uint32_t dv = off[v + 1] - off[v];
+        if (dv > kTcSearchMax) {
+          kind = dv > kTcWarpMax ? 1 : 0;
+          x = (1ull << kTcWorkBits) + (wp[e] - wp[b]) / kTcUnit + 1;
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kTcKinds; k++) {
+      if (!__any_sync(FULL, kind == k)) continue;
+      const unsigned long long mine = kind == k ? x : 0ull;
+      unsigned long long incl = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long t = __shfl_up_sync(FULL, incl, o);
+        if (lane >= o) incl += t;
+      }
+      unsigned long long base = 0;
+      if (lane == 31) base = atomicAdd(&ctl->size[k], incl);
+      base = __shfl_sync(FULL, base, 31) + incl - mine;
+      if (kind == k) {
+        const TcList& l = k ? block_list : warp_list;
+        const uint32_t i = (uint32_t)(base >> kTcWorkBits);
+        l.rank[i] = (uint32_t)r;
+        l.at[i] = base & ((1ull << kTcWorkBits) - 1);
+      }
+    }
   }
 }
 
-// Item k of rank r starts at the first entry whose probes begin at or after
-// k * kTcWork (counted from the list's start) and ends where the next begins.
-__global__ void item_fill_k(const uint32_t* __restrict__ first, const uint32_t* __restrict__ in_off,
-                            const uint32_t* __restrict__ off, const uint32_t* __restrict__ vertex_of,
-                            const uint64_t* __restrict__ wp, uint64_t n,
-                            uint32_t* __restrict__ item_rank, uint32_t* __restrict__ item_begin,
-                            uint32_t* __restrict__ item_end) {
-  for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n;
-       r += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t q0 = first[r], q1 = first[r + 1];
-    if (q0 == q1) continue;
-    const uint32_t lo = in_off[r], hi = in_off[r + 1];
-    const uint32_t v = vertex_of[r];
-    const uint64_t unit = off[v + 1] - off[v] > kTcWarpMax ? kTcWork * kTcBlockWarps : kTcWork;
-    const uint64_t base = wp[lo];
-    uint32_t prev = lo;
-    for (uint32_t q = q0; q < q1; q++) {
-      uint32_t e = hi;
-      if (q + 1 < q1) {  // first entry whose probes start at or after the next cut
-        const uint64_t cut = base + (uint64_t)(q + 1 - q0) * unit;
-        uint32_t a = prev, b = hi;
-        while (a < b) {
-          const uint32_t mid = (a + b) >> 1;
-          if (wp[mid] < cut) a = mid + 1; else b = mid;
-        }
-        e = a;
-      }
-      item_rank[q] = (uint32_t)r;
-      item_begin[q] = prev;
-      item_end[q] = e;
-      prev = e;
+// Chunk c of a kind starts c * step units into its list's work: in the last
+// vertex that starts at or before, at the first entry whose probes begin at
+// or after.
+__global__ void tc_chunks_k(const uint32_t* __restrict__ in_off, const uint64_t* __restrict__ wp,
+                            TcList list, int kind, uint64_t min_work,
+                            uint64_t max_chunks, TcCtl* ctl) {
+  const unsigned long long size = ctl->size[kind];
+  const uint32_t count = (uint32_t)(size >> kTcWorkBits);
+  const uint64_t work = size & ((1ull << kTcWorkBits) - 1);
+  const uint64_t step = max(min_work, (work + max_chunks - 1) / max_chunks);
+  const uint32_t used = (uint32_t)((work + step - 1) / step);
+  if (blockIdx.x == 0 && threadIdx.x == 0) ctl->chunks[kind] = used;
+  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c <= used; c += gridDim.x * blockDim.x) {
+    if (c == used) {
+      list.chunk_i[c] = count;
+      list.chunk_e[c] = 0;
+      continue;
     }
+    const uint64_t want = c * step;
+    uint32_t lo = 0, hi = count;
+    while (hi - lo > 1) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (list.at[mid] <= want) lo = mid; else hi = mid;
+    }
+    const uint32_t r = list.rank[lo];
+    uint32_t e = in_off[r], end = in_off[r + 1];
+    const uint64_t cut = wp[e] + (want - list.at[lo]) * kTcUnit;
+    while (e < end) {
+      const uint32_t mid = e + ((end - e) >> 1);
+      if (wp[mid] < cut) e = mid + 1; else end = mid;
+    }
+    list.chunk_i[c] = lo;
+    list.chunk_e[c] = e;
   }
 }
 
@@ -636,40 +836,44 @@ void triangle_count_run(TopoImpl* t, uint32_t* d_tri, cudaStream_t s) {
   // in-lists: the oriented edges grouped by target rank (sources in row
   // order), then the rows re-sorted by target rank (a stable sort of the
   // in-list order by source), and each in-list entry's slot in its sorted row
-  Scratch<uint32_t> in_off(n + 1, s), in_src(mo, s), in_pos(mo, s);
+  Scratch<uint32_t> in_off(n + 1, s), in_src(mo, s), in_pos(mo, s), in_rank(mo, s);
   {
-    Scratch<uint32_t> keys(mo, s);
-    radix_sort_pairs(o_tgt.get(), o_src.get(), mo, bits_for(n - 1), keys.get(), in_src.get(),
+    uint32_t* const keys = in_rank.get();
+    radix_sort_pairs(o_tgt.get(), o_src.get(), mo, bits_for(n - 1), keys, in_src.get(),
                      nullptr, nullptr, s);
-    offsets_from_sorted(keys.get(), mo, n, in_off.get(), s);
+    offsets_from_sorted(keys, mo, n, in_off.get(), s);
     Scratch<uint32_t> rows(mo, s), order(mo, s);
     radix_sort_pairs(in_src.get(), nullptr, mo, bits_for(n - 1), rows.get(), order.get(),
-                     keys.get(), o_tgt.get(), s);
+                     keys, o_tgt.get(), s);
     pos_scatter_k<<<grid_for(mo), kBlock, 0, s>>>(order.get(), mo, in_pos.get());
     UG_LAUNCH_CHECK();
   }
   o_src.release();
-  // work items, by rank ascending, of about kTcWork probes each
+  // chunks of equal probes over the lists of vertices that take a table
   Scratch<uint64_t> wp(mo + 1, s);
   entry_work_k<<<grid_for(mo), kBlock, 0, s>>>(o_off.get(), in_src.get(), in_pos.get(), mo,
                                                wp.get());
   UG_LAUNCH_CHECK();
   UG_CUDA(cudaMemsetAsync(wp.get() + mo, 0, sizeof(uint64_t), s));
   exclusive_scan_u64(wp.get(), wp.get(), mo + 1, nullptr, s);
-  Scratch<uint32_t> item_first(n + 1, s);
-  item_count_k<<<grid_for(n), kBlock, 0, s>>>(in_off.get(), o_off.get(), vertex_of.get(), wp.get(),
-                                               n, item_first.get());
+  const uint64_t listed = std::min<uint64_t>(n, mo / kTcSearchMax + 1);  // at most, of a kind
+  Scratch<uint32_t> ranks(kTcKinds * listed, s), chunk_at(2 * (kTcChunks[0] + kTcChunks[1] + 2ull), s);
+  Scratch<uint64_t> before(kTcKinds * listed, s);
+  Scratch<TcCtl> ctl(1, s);
+  UG_CUDA(cudaMemsetAsync(ctl.get(), 0, sizeof(TcCtl), s));
+  TcList lists[kTcKinds];
+  for (int k = 0; k < kTcKinds; k++) {
+    uint32_t* at = chunk_at.get() + (k ? 2 * (kTcChunks[0] + 1ull) : 0);
+    lists[k] = TcList{ranks.get() + k * listed, before.get() + k * listed, at, at + kTcChunks[k] + 1};
+  }
+  tc_lists_k<<<grid_for(n), kBlock, 0, s>>>(in_off.get(), o_off.get(), vertex_of.get(), wp.get(), n,
+                                            lists[0], lists[1], ctl.get());
   UG_LAUNCH_CHECK();
-  UG_CUDA(cudaMemsetAsync(item_first.get() + n, 0, sizeof(uint32_t), s));
-  exclusive_scan_u32(item_first.get(), item_first.get(), n + 1, nullptr, s);
-  const uint32_t n_items = read_u32(item_first.get() + n, s);
-  if (n_items == 0) return;
-  Scratch<uint32_t> item_rank(n_items, s), item_begin(n_items, s), item_end(n_items, s);
-  item_fill_k<<<grid_for(n), kBlock, 0, s>>>(item_first.get(), in_off.get(), o_off.get(),
-                                              vertex_of.get(), wp.get(), n,
-                                              item_rank.get(), item_begin.get(), item_end.get());
-  UG_LAUNCH_CHECK();
-  wp.release();
+  for (int k = 0; k < kTcKinds; k++) {
+    tc_chunks_k<<<grid_for(kTcChunks[k] + 1), kBlock, 0, s>>>(in_off.get(), wp.get(), lists[k], k,
+                                                              kTcMinWork[k], kTcChunks[k], ctl.get());
+    UG_LAUNCH_CHECK();
+  }
   uint32_t max_dv = 0;
   {
     Scratch<unsigned> mx(1, s);
@@ -678,59 +882,58 @@ void triangle_count_run(TopoImpl* t, uint32_t* d_tri, cudaStream_t s) {
     UG_LAUNCH_CHECK();
     max_dv = read_u32(mx.get(), s);
   }
-  Scratch<unsigned long long> next(1, s);
   TcArgs a;
   a.off = o_off.get();
   a.tgt = o_tgt.get();
   a.in_off = in_off.get();
   a.in_src = in_src.get();
   a.in_pos = in_pos.get();
+  a.in_rank = in_rank.get();
   a.vertex_of = vertex_of.get();
-  a.item_rank = item_rank.get();
-  a.item_begin = item_begin.get();
-  a.item_end = item_end.get();
-  a.n_items = n_items;
+  a.entries = mo;
+  a.list = lists[0];
+  a.kind = 0;
+  a.ctl = ctl.get();
   a.tri = d_tri;
-  a.next = next.get();
-  constexpr int kSmallSlots = 2 * kTcWarpMax, kMidSlots = 2048, kWarpsW = 8, kWarpsB = kTcBlockWarps;
-  {  // |N+(v)| <= 256: a warp per item
+  {  // |N+(v)| <= 32: searched
+    static std::mutex mu;
+    static int cache[64] = {0};
+    const int per_sm = tc_blocks_per_sm(tc_middle_search_k, 256, 0, dev, cache, mu);
+    const uint64_t warps = 8ull * per_sm * sm_count(dev);
+    a.grab = (uint32_t)std::min<uint64_t>(kTcSearchEntries, (mo / (4 * warps) + 31) / 32 * 32 + 32);
+    tc_middle_search_k<<<per_sm * sm_count(dev), 256, 0, s>>>(a);
+    UG_LAUNCH_CHECK();
+    count_launch();
+  }
+  constexpr int kSmallSlots = 2 * kTcWarpMax, kWarpsW = 8, kWarpsB = kTcBlockWarps;
+  if (max_dv > kTcSearchMax) {  // up to 256: a warp per chunk
     static std::mutex mu;
     static int cache[64] = {0};
     const size_t smem = ((size_t)kWarpsW * 2 * kSmallSlots + kWarpsW * 32) * sizeof(uint32_t);
     const int per_sm = tc_blocks_per_sm(tc_middle_warp_k<kSmallSlots, kWarpsW>, kWarpsW * 32, smem,
                                         dev, cache, mu);
-    a.lo = 0;
-    a.hi = kSmallSlots / 2;
-    UG_CUDA(cudaMemsetAsync(a.next, 0, sizeof(unsigned long long), s));
     tc_middle_warp_k<kSmallSlots, kWarpsW><<<per_sm * sm_count(dev), kWarpsW * 32, smem, s>>>(a);
     UG_LAUNCH_CHECK();
     count_launch();
   }
-  if (max_dv > (uint32_t)kSmallSlots / 2) {  // up to 1,024: a block per item, table in shared memory
+  a.list = lists[1];
+  a.kind = 1;
+  Scratch<uint32_t> table;
+  if (max_dv > (uint32_t)kSmallSlots / 2) {  // above: a block per chunk
     static std::mutex mu;
     static int cache[64] = {0};
-    const size_t smem = (size_t)2 * kMidSlots * sizeof(uint32_t);
+    const size_t smem = (size_t)2 * kTcMidSlots * sizeof(uint32_t);
     const int per_sm = tc_blocks_per_sm(tc_middle_block_k<kWarpsB>, kWarpsB * 32, smem, dev, cache, mu);
-    a.lo = kSmallSlots / 2;
-    a.hi = kMidSlots / 2;
-    UG_CUDA(cudaMemsetAsync(a.next, 0, sizeof(unsigned long long), s));
-    tc_middle_block_k<kWarpsB><<<per_sm * sm_count(dev), kWarpsB * 32, smem, s>>>(a, nullptr, kMidSlots);
-    UG_LAUNCH_CHECK();
-    count_launch();
-  }
-  if (max_dv > (uint32_t)kMidSlots / 2) {  // above: a block per item, table in global memory
+    const unsigned blocks = (unsigned)(per_sm * sm_count(dev));
     uint32_t slots = 1;
     while (slots < 2ull * max_dv) slots <<= 1;
-    const unsigned blocks = 2u * (unsigned)sm_count(dev);
-    Scratch<uint32_t> table((size_t)blocks * 2 * slots, s);
-    // keys empty (all ones), counts zero
-    fill_tables_k<<<grid_for((uint64_t)blocks * 2 * slots), kBlock, 0, s>>>(table.get(), blocks,
-                                                                              slots);
-    UG_LAUNCH_CHECK();
-    a.lo = kMidSlots / 2;
-    a.hi = 0xFFFFFFFFu;
-    UG_CUDA(cudaMemsetAsync(a.next, 0, sizeof(unsigned long long), s));
-    tc_middle_block_k<kWarpsB><<<blocks, kWarpsB * 32, 0, s>>>(a, table.get(), slots);
+    if (max_dv > kTcMidSlots / 2) {  // keys empty (all ones), counts zero
+      table.alloc((size_t)blocks * 2 * slots, s);
+      fill_tables_k<<<grid_for((uint64_t)blocks * 2 * slots), kBlock, 0, s>>>(table.get(), blocks,
+                                                                                slots);
+      UG_LAUNCH_CHECK();
+    }
+    tc_middle_block_k<kWarpsB><<<blocks, kWarpsB * 32, smem, s>>>(a, table.get(), slots);
     UG_LAUNCH_CHECK();
     count_launch();
   }
