@@ -1553,6 +1553,10 @@ void pagerank_run(TopoImpl* t, const ursa_gpu_pagerank_params& p, const double* 
   if (stats) *stats = ursa_gpu_pagerank_stats{0, 0.0, 0.0};
   if (n == 0) return;
   const bool weighted = d_weights != nullptr;
+  if (!weighted && pagerank_small_fits(t)) {
+    pagerank_small_run(t, p, d_out, s, stats);
+    return;
+  }
   PrPlan* plan = ensure_pr_plan(t, s, weighted);
   const int G = weighted ? pr_grid<true>(t->device) : pr_grid<false>(t->device);
   const size_t smem = pr_smem_bytes();

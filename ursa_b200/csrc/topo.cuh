@@ -87,6 +87,11 @@ void csr_owners(const uint32_t* off, uint64_t n, uint64_t m, uint32_t* owner, cu
 void degree_run(TopoImpl* t, int dir, uint32_t* d_out, cudaStream_t s);
 void pagerank_run(TopoImpl* t, const ursa_gpu_pagerank_params& p, const double* d_weights,
                   double* d_out, cudaStream_t s, ursa_gpu_pagerank_stats* stats);
+// The same for graphs that fit one thread-block cluster, unweighted
+// (pagerank_small.cu).
+bool pagerank_small_fits(const TopoImpl* t);
+void pagerank_small_run(TopoImpl* t, const ursa_gpu_pagerank_params& p, double* d_out, cudaStream_t s,
+                        ursa_gpu_pagerank_stats* stats);
 void cc_weak_run(TopoImpl* t, uint32_t* d_out, cudaStream_t s);
 void triangle_count_run(TopoImpl* t, uint32_t* d_tri, cudaStream_t s);
 void clustering_run(TopoImpl* t, double* d_out, cudaStream_t s);
