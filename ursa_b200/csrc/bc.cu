@@ -224,23 +224,31 @@ __global__ void fdeg_out_k(const uint32_t* __restrict__ off, const uint32_t* __r
 // ---- 64 sources at once (unweighted) -------------------------------------
 // Batch b holds sources [64 b, 64 b + 64) of the source list, the
 // reference's accumulation chunk (betweenness.rs:45-70).  Per node v the
-// batch keeps a row of 64 values per quantity (hop i32, sigma f64, delta
-// f64; node-major, so lane j of a warp reads entries j and j + 32 of a row
-// in one coalesced access), a visited mask and a frontier mask (bit q =
-// source q).
-//  forward level L: one warp per node v still missing some sources; it walks
-//    v's in-edges u -> v in CSR order (eight in flight); the sources in
-//    front[u] & need reach v at level L, sigma_q[v] += sigma_q[u] for each
-//    (per slot, as brandes_from counts parallel edges), and the slot of the
-//    out-CSR holding u -> v records those sources (dag[], the shortest-path
-//    DAG per source);
+// batch keeps a row of 64 f64 (node-major: lane l of a warp holds sources 2 l
+// and 2 l + 1, one 16-byte access), and per level a mask of the sources that
+// reach v there (bit q = source q).
+//  forward level L: one warp per node v still missing some sources; over v's
+//    in-edges u -> v in CSR order, the sources in front[u] & need reach v at
+//    level L, sigma_q[v] += sigma_q[u] for each (per slot, as brandes_from
+//    counts parallel edges);
 //  backward level L (deepest first): one warp per node v with some source at
-//    level L; over v's out-edges in CSR order, for each source q of dag[k]
-//    at level L, delta_q[v] += sigma_q[v] * ((1 + delta_q[w]) / sigma_q[w])
+//    level L; over v's out-edges v -> w in CSR order, an edge is on the
+//    shortest-path DAG of the sources in mask_L[v] & mask_L+1[w]:
+//    delta_q[v] = sigma_q[v] * the sum of c_q[w], c = (1 + delta) / sigma
 //    (reverse_accumulate, :81-98, summed per successor instead of per
-//    predecessor list);
+//    predecessor list); c_q[v] then takes the place of sigma_q[v], which
+//    nobody reads any more;
 //  fold: per node, the batch's partial = sum over q in source order of
 //    delta_q[v] (v != source q), added to the result in batch order.
+// What bounds it is the rows: 512 bytes per edge and level that lies on some
+// source's DAG, from HBM.  So a warp finds the edges with a source in common
+// first (32 at a time, 8-byte masks that stay in L2) and has eight rows in
+// flight; the masks per level take the place of a DAG mask per edge (a random
+// read-modify-write per edge in the forward pass) and of a hop per (node,
+// source), and c that of a second row and a division per edge and source.
+// 256 sources on a Poisson graph of a million nodes, 16.8M edges: forward
+// 15.8 ms against 37.4, backward 14.9 against 51.4; the two deep levels, where
+// most edges meet, move about 4 TB/s of rows each.
 constexpr int kBcB = 64;
 
 struct BcBatchArgs {
@@ -262,6 +270,326 @@ struct BcBatchArgs {
   unsigned* found;
 };
 
+constexpr int kBcRows = 8;            // rows in flight per warp (4: 41.3 ms a call, 8: 40.8, 16: 42.9)
+constexpr int kBcOcc = 4;             // blocks per SM: registers for those rows (3: 47.9 ms, 5: 42.4)
+constexpr uint32_t kBcLong = 1024;     // longer rows are walked by the whole block
+constexpr int kBcLongList = 32;        // ... as many as it can list; the rest by their warp
+constexpr int kBcWarps = kBlock / 32;
+constexpr uint32_t kBcNone = 0xFFFFFFFFu;
+constexpr uint32_t kBcGroup = 32;      // most nodes a warp takes at a time
+// Mask levels kept, in no more memory than a hop per (node, source) takes;
+// deeper searches (roads, chains) take bc_forward_k.
+constexpr size_t kBcMaxLevels = 32;
+
+struct BcLevelArgs {
+  const uint32_t* off;   // forward: the in-CSR; backward: the out-CSR
+  const uint32_t* adj;
+  uint64_t n;
+  uint64_t qmask;
+  uint64_t* vis;          // forward
+  const uint64_t* front;  // forward: masks of the last level; backward: of the next one
+  uint64_t* mask;         // this level's masks (forward: written)
+  double* row;            // n x 64: sigma, then c
+  double* delta;          // n x 64 (backward)
+  unsigned* found;
+  uint32_t group;         // nodes a warp takes at a time
+};
+
+// Two f64 of a row past L1, or zeros without the predicate.  Volatile, so that
+// a warp's eight loads are issued before the first sum waits for one.
+__device__ __forceinline__ double2 bc_load(const double* p, bool take) {
+  double2 r;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.u32 p, %3, 0;\n\t"
+      "mov.f64 %0, 0d0000000000000000;\n\t"
+      "mov.f64 %1, 0d0000000000000000;\n\t"
+      "@p ld.global.cg.v2.f64 {%0, %1}, [%2];\n\t}"
+      : "=d"(r.x), "=d"(r.y)
+      : "l"(p), "r"((uint32_t)take));
+  return r;
+}
+
+// A warp's list of the edges of a step that share a source: the neighbour and
+// the sources shared (two words: lanes 0..15 hold sources 0..31).
+struct BcStep {
+  uint32_t f[32 + kBcRows][2];
+  uint32_t u[32 + kBcRows];
+};
+
+// Adds, in order, the rows of a step of up to 32 edges (a lane each: the
+// neighbour u and the sources f it shares) into every lane's two sums.
+__device__ __forceinline__ void bc_add_step(BcStep& st, uint32_t u, uint64_t f, const double* row,
+                                            double2& sum) {
+  const uint32_t FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const uint32_t some = __ballot_sync(FULL, f != 0);
+  if (!some) return;
+  const int count = __popc(some);
+  if (f) {
+    const int at = __popc(some & ((1u << lane) - 1u));
+    st.f[at][0] = (uint32_t)f;
+    st.f[at][1] = (uint32_t)(f >> 32);
+    st.u[at] = u;
+  }
+  if (lane < kBcRows) st.f[count + lane][0] = st.f[count + lane][1] = 0;  // the last rows, unused
+  __syncwarp();
+  const int word = lane >> 4, shift = 2 * (lane & 15);
+  for (int j0 = 0; j0 < count; j0 += kBcRows) {
+    double2 r[kBcRows];
+    uint32_t bits[kBcRows];
+#pragma unroll
+    for (int j = 0; j < kBcRows; j++) {
+      bits[j] = (st.f[j0 + j][word] >> shift) & 3u;
+      r[j] = bc_load(row + (uint64_t)st.u[j0 + j] * kBcB + 2 * lane, bits[j] != 0);
+    }
+#pragma unroll
+    for (int j = 0; j < kBcRows; j++) {
+      sum.x = __dadd_rn(sum.x, bits[j] & 1u ? r[j].x : 0.0);
+      sum.y = __dadd_rn(sum.y, bits[j] & 2u ? r[j].y : 0.0);
+    }
+  }
+  __syncwarp();
+}
+
+// The same over adj[k], k in [b, e), for the sources in mask[adj[k]] & need;
+// adds the sources met to the lane's own `met`.
+__device__ __forceinline__ void bc_add_rows(BcStep& st, const uint32_t* __restrict__ adj,
+                                            const uint64_t* __restrict__ mask, const double* row,
+                                            uint32_t b, uint32_t e, uint64_t need, uint64_t& met,
+                                            double2& sum) {
+  const int lane = threadIdx.x & 31;
+  for (uint32_t k0 = b; k0 < e; k0 += 32) {
+    uint32_t u = 0;
+    uint64_t f = 0;
+    if (k0 + lane < e) {
+      u = adj[k0 + lane];
+      f = mask[u] & need;
+    }
+    met |= f;
+    bc_add_step(st, u, f, row, sum);
+  }
+}
+
+__device__ __forceinline__ uint64_t bc_or(uint64_t met) {
+  return ((uint64_t)__reduce_or_sync(0xffffffffu, (uint32_t)(met >> 32)) << 32) |
+         __reduce_or_sync(0xffffffffu, (uint32_t)met);
+}
+
+// A warp's nodes, one per lane: need (sources wanted, 0: nothing to do) and
+// edges [b, e) of each.  settle(l, need, met, sum) takes the result of lane
+// l's node, in lane order (met: per lane, to be ORed over the warp).  The
+// next node's neighbours are loaded while a node's rows are added.
+template <class Settle>
+__device__ __forceinline__ void bc_nodes(const BcLevelArgs& A, BcStep& st, uint64_t need, uint32_t b,
+                                         uint32_t e, Settle&& settle) {
+  const uint32_t FULL = 0xffffffffu;
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t todo = __ballot_sync(FULL, need != 0);
+  uint32_t u1 = kBcNone, b1 = 0, e1 = 0;
+  int l1 = -1;
+  auto next = [&]() {
+    l1 = __ffs(todo) - 1;  // -1 after the last
+    todo &= todo - 1;
+    b1 = __shfl_sync(FULL, b, l1 & 31);
+    e1 = l1 >= 0 ? __shfl_sync(FULL, e, l1 & 31) : b1;
+    u1 = lane < e1 - b1 ? A.adj[b1 + lane] : kBcNone;
+  };
+  next();
+  while (l1 >= 0) {
+    const int l = l1;
+    const uint32_t u = u1, lb = b1, le = e1;
+    const uint64_t ln = __shfl_sync(FULL, need, l);
+    const uint64_t f = u != kBcNone ? A.front[u] & ln : 0ull;
+    next();
+    uint64_t met = f;
+    double2 sum = make_double2(0.0, 0.0);
+    bc_add_step(st, u, f, A.row, sum);
+    if (le - lb > 32) bc_add_rows(st, A.adj, A.front, A.row, lb + 32, le, ln, met, sum);
+    settle(l, ln, met, sum);
+  }
+}
+
+// The same over one long row by every warp of the block: runs of 32-edge
+// steps per warp, combined in warp order; valid in warp 0.
+struct BcShared {
+  BcStep step[kBcWarps];
+  uint32_t list[kBcLongList];
+  unsigned count;
+  double2 sum[kBcWarps][32];
+  uint64_t met[kBcWarps];
+};
+__device__ __forceinline__ uint64_t bc_add_rows_block(BcShared& sh, const uint32_t* adj,
+                                                      const uint64_t* mask, const double* row,
+                                                      uint32_t b, uint32_t e, uint64_t need,
+                                                      double2& sum) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint32_t per = ((e - b + kBcWarps - 1) / kBcWarps + 31) / 32 * 32;
+  const uint32_t lo = min(e, b + w * per), hi = min(e, lo + per);
+  double2 part = make_double2(0.0, 0.0);
+  uint64_t met = 0;
+  bc_add_rows(sh.step[w], adj, mask, row, lo, hi, need, met, part);
+  met = bc_or(met);
+  sh.sum[w][lane] = part;
+  if (lane == 0) sh.met[w] = met;
+  __syncthreads();
+  uint64_t all = 0;
+  if (w == 0)
+    for (int i = 0; i < kBcWarps; i++) {
+      all |= sh.met[i];
+      sum.x = __dadd_rn(sum.x, sh.sum[i][lane].x);
+      sum.y = __dadd_rn(sum.y, sh.sum[i][lane].y);
+    }
+  __syncthreads();
+  return all;
+}
+
+__global__ void __launch_bounds__(kBlock, kBcOcc) bc_forward_level_k(BcLevelArgs A) {
+  __shared__ BcShared sh;
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) sh.count = 0;
+  __syncthreads();
+  const uint64_t gw = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  bool any = false;
+  auto settle = [&](uint64_t v, uint64_t reached, double2 sigma) {
+    if (!reached) return;
+    any = true;
+    if (lane == 0) {
+      A.mask[v] = reached;
+      A.vis[v] |= reached;
+    }
+    double* row = A.row + v * kBcB + 2 * lane;
+    const uint32_t bits = (uint32_t)(reached >> (2 * lane)) & 3u;
+    if (bits == 3u) {
+      *reinterpret_cast<double2*>(row) = sigma;
+    } else {
+      if (bits & 1u) row[0] = sigma.x;
+      if (bits & 2u) row[1] = sigma.y;
+    }
+  };
+  // lane l's node: nw apart, so that a run of long rows (the lowest ids of an
+  // R-MAT graph) is spread over the warps
+  for (uint64_t v0 = gw; v0 < A.n; v0 += nw * A.group) {
+    const uint64_t mine = v0 + lane * nw;
+    uint64_t need = 0;
+    uint32_t b = 0, e = 0;
+    if (lane < A.group && mine < A.n) {
+      A.mask[mine] = 0;
+      need = A.qmask & ~A.vis[mine];
+      if (need) {
+        b = A.off[mine];
+        e = A.off[mine + 1];
+      }
+      if (b == e) {
+        need = 0;
+      } else if (e - b > kBcLong) {
+        const unsigned at = atomicAdd(&sh.count, 1u);
+        if (at < kBcLongList) {
+          sh.list[at] = (uint32_t)mine;
+          need = 0;
+        }
+      }
+    }
+    __syncwarp();  // the cleared masks, before settle() sets one
+    bc_nodes(A, sh.step[threadIdx.x >> 5], need, b, e, [&](int l, uint64_t, uint64_t met, double2 sigma) {
+      if (__any_sync(0xffffffffu, met != 0)) settle(v0 + l * nw, bc_or(met), sigma);
+    });
+  }
+  __syncthreads();
+  const unsigned listed = min(sh.count, (unsigned)kBcLongList);
+  for (unsigned i = 0; i < listed; i++) {
+    const uint64_t v = sh.list[i];
+    double2 sigma = make_double2(0.0, 0.0);
+    const uint64_t reached = bc_add_rows_block(sh, A.adj, A.front, A.row, A.off[v], A.off[v + 1],
+                                               A.qmask & ~A.vis[v], sigma);
+    if (threadIdx.x < 32) settle(v, reached, sigma);
+  }
+  if (lane == 0 && any) atomicOr(A.found, 1u);
+}
+
+__global__ void __launch_bounds__(kBlock, kBcOcc) bc_backward_level_k(BcLevelArgs A) {
+  __shared__ BcShared sh;
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) sh.count = 0;
+  __syncthreads();
+  const uint64_t gw = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  auto settle = [&](uint64_t v, uint32_t bits, double2 c) {  // c: the sums of the successors' c
+    double* row = A.row + v * kBcB + 2 * lane;
+    double* delta = A.delta + v * kBcB + 2 * lane;
+    if (bits & 1u) {
+      const double sigma = row[0], d = __dmul_rn(sigma, c.x);
+      delta[0] = d;
+      row[0] = __ddiv_rn(__dadd_rn(1.0, d), sigma);
+    }
+    if (bits & 2u) {
+      const double sigma = row[1], d = __dmul_rn(sigma, c.y);
+      delta[1] = d;
+      row[1] = __ddiv_rn(__dadd_rn(1.0, d), sigma);
+    }
+  };
+  for (uint64_t v0 = gw; v0 < A.n; v0 += nw * A.group) {
+    const uint64_t mine = v0 + lane * nw;
+    uint64_t here = 0;
+    uint32_t b = 0, e = 0;
+    if (lane < A.group && mine < A.n) {
+      here = A.mask[mine];
+      if (here) {
+        b = A.off[mine];
+        e = A.off[mine + 1];
+        if (e - b > kBcLong) {
+          const unsigned at = atomicAdd(&sh.count, 1u);
+          if (at < kBcLongList) {
+            sh.list[at] = (uint32_t)mine;
+            here = 0;
+          }
+        }
+      }
+    }
+    bc_nodes(A, sh.step[threadIdx.x >> 5], here, b, e, [&](int l, uint64_t at, uint64_t, double2 d) {
+      settle(v0 + l * nw, (uint32_t)(at >> (2 * lane)) & 3u, d);
+    });
+  }
+  __syncthreads();
+  const unsigned listed = min(sh.count, (unsigned)kBcLongList);
+  for (unsigned i = 0; i < listed; i++) {
+    const uint64_t v = sh.list[i];
+    const uint64_t here = A.mask[v];
+    double2 d = make_double2(0.0, 0.0);
+    bc_add_rows_block(sh, A.adj, A.front, A.row, A.off[v], A.off[v + 1], here, d);
+    if (threadIdx.x < 32) settle(v, (uint32_t)(here >> (2 * lane)) & 3u, d);
+  }
+}
+
+__global__ void bc_seed_level_k(const uint32_t* __restrict__ src, uint32_t nq, uint64_t* vis,
+                                uint64_t* mask, double* sigma) {
+  const uint32_t q = threadIdx.x;
+  if (q >= nq) return;
+  const uint32_t s = src[q];
+  atomicOr((unsigned long long*)(vis + s), 1ull << q);
+  atomicOr((unsigned long long*)(mask + s), 1ull << q);
+  sigma[(uint64_t)s * kBcB + q] = 1.0;
+}
+
+// The batch's partial (sources in order, each source's own node excluded),
+// added to out in batch order; vis: the sources that reach each node.
+__global__ void bc_fold_level_k(const double* __restrict__ delta, const uint64_t* __restrict__ vis,
+                                const uint32_t* __restrict__ src, uint32_t nq, uint64_t n,
+                                double* __restrict__ out) {
+  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n;
+       v += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t met = vis[v];
+    if (!met) continue;
+    double p = 0.0;
+    for (uint32_t q = 0; q < nq; q++)
+      if (((met >> q) & 1ull) && src[q] != v) p = __dadd_rn(p, delta[v * kBcB + q]);
+    out[v] = __dadd_rn(out[v], p);
+  }
+}
+
+// ---- searches deeper than kBcMaxLevels: the same batch with a hop per (node,
+// source) and, per out-slot, a mask of the sources whose DAG holds the edge
 __global__ void bc_seed_k(const uint32_t* __restrict__ src, uint32_t nq, uint64_t* vis, uint64_t* front,
                           int32_t* hop, double* sigma) {
   const uint32_t q = threadIdx.x;
@@ -579,11 +907,11 @@ __global__ void compose_k(const uint32_t* __restrict__ a, const uint32_t* __rest
 
 }  // namespace
 
-// Unweighted betweenness over `sources`, 64 at a time, added into d_out.
-static void betweenness_batched(TopoImpl* t, const std::vector<uint32_t>& sources, double* d_out,
-                                cudaStream_t s) {
+// Unweighted betweenness over d_src (at most 64 sources), added into d_out,
+// with a hop per (node, source): any depth.  The three buffers are scratch.
+static void betweenness_deep(TopoImpl* t, const uint32_t* d_src, uint32_t nq, uint64_t* vis,
+                             double* sigma, double* delta, double* d_out, cudaStream_t s) {
   const uint64_t n = t->n, m = t->m;
-  ensure_in(t, s);
   Scratch<uint32_t> in_to_out(m ? m : 1, s);
   if (m) {
     Scratch<uint32_t> inv(m, s);
@@ -592,10 +920,8 @@ static void betweenness_batched(TopoImpl* t, const std::vector<uint32_t>& source
     compose_k<<<grid_for(m), kBlock, 0, s>>>(t->in.eid.get(), inv.get(), m, in_to_out.get());
     UG_LAUNCH_CHECK();
   }
-  Scratch<uint64_t> vis(n, s), fa(n, s), fb(n, s), dag(m ? m : 1, s);
+  Scratch<uint64_t> fa(n, s), fb(n, s), dag(m ? m : 1, s);
   Scratch<int32_t> hop(n * kBcB, s);
-  Scratch<double> sigma(n * kBcB, s), delta(n * kBcB, s);
-  Scratch<uint32_t> d_src(kBcB, s);
   Scratch<unsigned> found(1, s);
   BcBatchArgs a;
   a.in_off = t->in.off.get();
@@ -604,49 +930,108 @@ static void betweenness_batched(TopoImpl* t, const std::vector<uint32_t>& source
   a.out_off = t->out.off.get();
   a.out_tgt = t->out.tgt.get();
   a.n = n;
-  a.vis = vis.get();
+  a.vis = vis;
   a.hop = hop.get();
-  a.sigma = sigma.get();
-  a.delta = delta.get();
+  a.sigma = sigma;
+  a.delta = delta;
   a.dag = dag.get();
   a.found = found.get();
+  a.qmask = nq == 64 ? ~0ull : ((1ull << nq) - 1ull);
   const unsigned gw = grid_for(n * 32, kBlock, 148u * 8u);
+  UG_CUDA(cudaMemsetAsync(vis, 0, n * 8, s));
+  UG_CUDA(cudaMemsetAsync(fa.get(), 0, n * 8, s));
+  UG_CUDA(cudaMemsetAsync(hop.get(), 0xFF, n * kBcB * 4, s));
+  UG_CUDA(cudaMemsetAsync(sigma, 0, n * kBcB * 8, s));
+  UG_CUDA(cudaMemsetAsync(delta, 0, n * kBcB * 8, s));
+  if (m) UG_CUDA(cudaMemsetAsync(dag.get(), 0, m * 8, s));
+  bc_seed_k<<<1, kBcB, 0, s>>>(d_src, nq, vis, fa.get(), hop.get(), sigma);
+  UG_LAUNCH_CHECK();
+  int32_t L = 0;
+  uint64_t* cur = fa.get();
+  uint64_t* nxt = fb.get();
+  while (true) {
+    a.level = L + 1;
+    a.front = cur;
+    a.next = nxt;
+    UG_CUDA(cudaMemsetAsync(found.get(), 0, 4, s));
+    bc_forward_k<<<gw, kBlock, 0, s>>>(a);
+    UG_LAUNCH_CHECK();
+    if (!read_u32(found.get(), s)) break;
+    L++;
+    std::swap(cur, nxt);
+  }
+  // nodes of the deepest level L have no successors (delta 0)
+  for (int32_t lvl = L - 1; lvl >= 0; lvl--) {
+    a.level = lvl;
+    bc_backward_k<<<gw, kBlock, 0, s>>>(a);
+    UG_LAUNCH_CHECK();
+  }
+  bc_fold_k<<<grid_for(n), kBlock, 0, s>>>(delta, d_src, nq, n, d_out);
+  UG_LAUNCH_CHECK();
+}
+
+// Unweighted betweenness over `sources`, 64 at a time, added into d_out.
+static void betweenness_batched(TopoImpl* t, const std::vector<uint32_t>& sources, double* d_out,
+                                cudaStream_t s) {
+  const uint64_t n = t->n;
+  ensure_in(t, s);
+  Scratch<uint64_t> vis(n, s);
+  Scratch<double> row(n * kBcB, s), delta(n * kBcB, s);
+  Scratch<uint32_t> d_src(kBcB, s);
+  Scratch<unsigned> found(1, s);
+  std::vector<Scratch<uint64_t>> masks;  // masks[l]: the sources that reach each node at level l
+  auto level = [&](size_t l) {
+    while (masks.size() <= l) masks.emplace_back(n, s);
+    return masks[l].get();
+  };
+  BcLevelArgs a{};
+  a.n = n;
+  a.vis = vis.get();
+  a.row = row.get();
+  a.delta = delta.get();
+  a.found = found.get();
+  bool deep = false;  // the graph has searches past the levels kept
+  const unsigned gw = grid_for(n * 32, kBlock, 148u * kBcOcc);
+  // few nodes at a time while there are fewer than four groups per warp
+  a.group = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(kBcGroup, n / (4ull * gw * kBcWarps)));
   for (size_t c0 = 0; c0 < sources.size(); c0 += kBcB) {
     const uint32_t nq = (uint32_t)std::min<size_t>(kBcB, sources.size() - c0);
     a.qmask = nq == 64 ? ~0ull : ((1ull << nq) - 1ull);
     UG_CUDA(cudaMemcpyAsync(d_src.get(), sources.data() + c0, nq * 4, cudaMemcpyHostToDevice, s));
     UG_CUDA(cudaMemsetAsync(vis.get(), 0, n * 8, s));
-    UG_CUDA(cudaMemsetAsync(fa.get(), 0, n * 8, s));
-    UG_CUDA(cudaMemsetAsync(hop.get(), 0xFF, n * kBcB * 4, s));
-    UG_CUDA(cudaMemsetAsync(sigma.get(), 0, n * kBcB * 8, s));
-    UG_CUDA(cudaMemsetAsync(delta.get(), 0, n * kBcB * 8, s));
-    if (m) UG_CUDA(cudaMemsetAsync(dag.get(), 0, m * 8, s));
-    bc_seed_k<<<1, kBcB, 0, s>>>(d_src.get(), nq, vis.get(), fa.get(), hop.get(), sigma.get());
+    UG_CUDA(cudaMemsetAsync(level(0), 0, n * 8, s));
+    bc_seed_level_k<<<1, kBcB, 0, s>>>(d_src.get(), nq, vis.get(), level(0), row.get());
     UG_LAUNCH_CHECK();
-    int32_t L = 0;
-    uint64_t* cur = fa.get();
-    uint64_t* nxt = fb.get();
-    while (true) {
-      a.level = L + 1;
-      a.front = cur;
-      a.next = nxt;
+    a.off = t->in.off.get();
+    a.adj = t->in.tgt.get();
+    size_t L = 0;  // the deepest level met
+    while (!deep) {
+      if (L + 1 >= kBcMaxLevels) {
+        deep = true;
+        break;
+      }
+      a.front = level(L);
+      a.mask = level(L + 1);
       UG_CUDA(cudaMemsetAsync(found.get(), 0, 4, s));
-      bc_forward_k<<<gw, kBlock, 0, s>>>(a);
+      bc_forward_level_k<<<gw, kBlock, 0, s>>>(a);
       UG_LAUNCH_CHECK();
-      unsigned f = 0;
-      UG_CUDA(cudaMemcpyAsync(&f, found.get(), 4, cudaMemcpyDeviceToHost, s));
-      UG_CUDA(cudaStreamSynchronize(s));
-      if (!f) break;
+      if (!read_u32(found.get(), s)) break;
       L++;
-      std::swap(cur, nxt);
     }
-    // nodes of the deepest level L have no successors (delta 0)
-    for (int32_t lvl = L - 1; lvl >= 0; lvl--) {
-      a.level = lvl;
-      bc_backward_k<<<gw, kBlock, 0, s>>>(a);
+    if (deep) {
+      masks.clear();
+      betweenness_deep(t, d_src.get(), nq, vis.get(), row.get(), delta.get(), d_out, s);
+      continue;
+    }
+    a.off = t->out.off.get();
+    a.adj = t->out.tgt.get();
+    for (size_t l = L; l >= 1; l--) {  // level 0, the sources, takes no part in the result
+      a.mask = level(l);
+      a.front = level(l + 1);
+      bc_backward_level_k<<<gw, kBlock, 0, s>>>(a);
       UG_LAUNCH_CHECK();
     }
-    bc_fold_k<<<grid_for(n), kBlock, 0, s>>>(delta.get(), d_src.get(), nq, n, d_out);
+    bc_fold_level_k<<<grid_for(n), kBlock, 0, s>>>(delta.get(), vis.get(), d_src.get(), nq, n, d_out);
     UG_LAUNCH_CHECK();
   }
 }
