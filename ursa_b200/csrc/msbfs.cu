@@ -43,7 +43,18 @@ namespace {
 
 constexpr int kMsBlock = 256;
 constexpr int kMsWarps = kMsBlock / 32;
-constexpr uint64_t kMsSourcesPerLaunch = 1024;
+constexpr int kMsOcc = 4;   // blocks per SM of the 256-source kernel (64 registers; 5 would spill)
+constexpr int kMsOcc1 = 5;  // ... of the 64-source kernel (48)
+constexpr uint64_t kMsSourcesPerLaunch = 1024;  // per group
+// A level of a small graph is too little work for the grid: on R-MAT-16 78%
+// of the warps' time was the wait at the level's barrier.  So the grid is cut
+// into groups of blocks, each with its own barrier and masks and every
+// groups-th batch: while one group waits, another one's blocks work.  R-MAT-16
+// from every node with 1 / 6 / 16 / 32 / 64 groups: 89.6 / 46.0 / 34.4 / 27.3 /
+// 20.7 ms; beyond that the masks (4 x 32 bytes a node and group) leave L2.
+constexpr uint64_t kMsGroups = 128;       // at most
+constexpr uint64_t kMsNodesPerBlock = 8192;  // at most, of a group's pass
+constexpr uint64_t kMsMaskBytes = 512ull << 20;  // of all groups
 constexpr uint64_t kMsWaitNs = 5000000000ull;  // one grid-barrier wait
 constexpr uint64_t kMsPushDiv = 8;  // push while the frontier's out-edges are below m / 8
 constexpr uint32_t kMsHub = 64;    // in-degree above which a node's scan is split
@@ -155,8 +166,9 @@ struct MsArgs {
   unsigned long long* reach;
   unsigned long long* dsum;
   uint32_t* maxd;
-  unsigned* bar;  // grid barrier count, generation
+  unsigned* bar;  // per group: barrier count, generation
   int* err;
+  uint32_t groups, group_blocks;  // the grid: groups x group_blocks blocks
 };
 
 // Top-down half of a level: every frontier node v ORs its mask into acc[w]
@@ -274,8 +286,10 @@ __device__ __forceinline__ void ms_hub_chunk(const MsArgs& a, const unsigned lon
   if (y) atomicOr(&a.hacc[(uint64_t)h * W + lane], y);
 }
 
-template <int W>
-__global__ void __launch_bounds__(kMsBlock) ms_persist_k(MsArgs a) {
+// kGroups: the grid is cut into groups (else it is one, and the group index
+// costs no registers).
+template <int W, bool kGroups>
+__global__ void __launch_bounds__(kMsBlock, W == 4 ? kMsOcc : kMsOcc1) ms_persist_k(MsArgs a) {
   constexpr int S = 64 * W;     // sources per batch
   constexpr int R = 64 * W + 8;  // counter row length
   static_assert(S <= kMsBlock, "one thread per source of a batch");
@@ -284,11 +298,21 @@ __global__ void __launch_bounds__(kMsBlock) ms_persist_k(MsArgs a) {
   __shared__ unsigned s_act[2 * W];
   const int lane = threadIdx.x & 31;
   const uint64_t n = a.n;
-  const uint64_t nwarps = (uint64_t)gridDim.x * kMsWarps;
-  const uint64_t gwarp = (uint64_t)blockIdx.x * kMsWarps + (threadIdx.x >> 5);
-  const uint64_t nthreads = (uint64_t)gridDim.x * blockDim.x;
-  const uint64_t gtid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  for (uint64_t bt = a.b_begin; bt < a.b_end; bt++) {
+  const uint32_t group = kGroups ? blockIdx.x / a.group_blocks : 0;
+  const uint32_t block = kGroups ? blockIdx.x % a.group_blocks : blockIdx.x;
+  if (!kGroups) a.group_blocks = gridDim.x;
+  a.visited += group * n * W;
+  a.fr0 += group * n * W;
+  a.fr1 += group * n * W;
+  a.acc += group * n * W;
+  a.hacc += group * a.n_hubs * W;
+  a.count += group * 3 * R;
+  a.bar += group * 2;
+  const uint64_t nwarps = (uint64_t)a.group_blocks * kMsWarps;
+  const uint64_t gwarp = (uint64_t)block * kMsWarps + (threadIdx.x >> 5);
+  const uint64_t nthreads = (uint64_t)a.group_blocks * blockDim.x;
+  const uint64_t gtid = (uint64_t)block * blockDim.x + threadIdx.x;
+  for (uint64_t bt = a.b_begin + group; bt < a.b_end; bt += kGroups ? a.groups : 1) {
     const uint64_t s0 = bt * S;
     const uint64_t left = a.n_sources - s0;
     const uint32_t k = left < (uint64_t)S ? (uint32_t)left : (uint32_t)S;
@@ -302,9 +326,9 @@ __global__ void __launch_bounds__(kMsBlock) ms_persist_k(MsArgs a) {
       a.visited[x] = 0;
       a.fr0[x] = 0;
     }
-    grid_barrier(a.bar, a.bar + 1, gridDim.x, a.err, kMsWaitNs);
+    grid_barrier(a.bar, a.bar + 1, a.group_blocks, a.err, kMsWaitNs);
     if (*(volatile int*)a.err) return;
-    if (blockIdx.x == 0) {  // every block has read the previous batch's last counter row
+    if (block == 0) {  // every block has read the previous batch's last counter row
       for (int x = threadIdx.x; x < 3 * R; x += kMsBlock) a.count[x] = 0;
       __syncthreads();
       if (threadIdx.x < k) {
@@ -316,7 +340,7 @@ __global__ void __launch_bounds__(kMsBlock) ms_persist_k(MsArgs a) {
         if (a.dist) a.dist[(s0 + threadIdx.x) * n + src] = 0;
       }
     }
-    grid_barrier(a.bar, a.bar + 1, gridDim.x, a.err, kMsWaitNs);
+    grid_barrier(a.bar, a.bar + 1, a.group_blocks, a.err, kMsWaitNs);
     if (*(volatile int*)a.err) return;
     unsigned long long reach = 0, dsum = 0;  // block 0, thread b < k: source s0 + b
     uint32_t maxd = 0;
@@ -329,12 +353,12 @@ __global__ void __launch_bounds__(kMsBlock) ms_persist_k(MsArgs a) {
       for (int x = threadIdx.x; x < S; x += kMsBlock) sc[x] = 0;
       if (threadIdx.x == 0) s_mf = 0;
       // row (level + 1) % 3 was last read before the previous barrier
-      if (blockIdx.x == 0)
+      if (block == 0)
         for (int x = threadIdx.x; x < R; x += kMsBlock) a.count[((level + 1) % 3) * R + x] = 0;
       __syncthreads();
       if (push) {
         ms_push<W>(a, cur, gwarp, nwarps, lane);
-        grid_barrier(a.bar, a.bar + 1, gridDim.x, a.err, kMsWaitNs);
+        grid_barrier(a.bar, a.bar + 1, a.group_blocks, a.err, kMsWaitNs);
         if (*(volatile int*)a.err) return;
       }
       if (!push)
@@ -409,7 +433,7 @@ __global__ void __launch_bounds__(kMsBlock) ms_persist_k(MsArgs a) {
       }
       if (!push && a.n_hubs) {
         // hubs: their chunks' ORs are all in hacc after the barrier
-        grid_barrier(a.bar, a.bar + 1, gridDim.x, a.err, kMsWaitNs);
+        grid_barrier(a.bar, a.bar + 1, a.group_blocks, a.err, kMsWaitNs);
         if (*(volatile int*)a.err) return;
         for (uint64_t i0 = gwarp * 32; i0 < a.n_hubs; i0 += nwarps * 32) {
           const uint64_t i = i0 + lane;
@@ -431,11 +455,11 @@ __global__ void __launch_bounds__(kMsBlock) ms_persist_k(MsArgs a) {
       for (int x = threadIdx.x; x < S; x += kMsBlock)
         if (sc[x]) atomicAdd(&row[x], (unsigned long long)sc[x]);
       if (threadIdx.x == 0 && s_mf) atomicAdd(&row[S], s_mf);
-      grid_barrier(a.bar, a.bar + 1, gridDim.x, a.err, kMsWaitNs);
+      grid_barrier(a.bar, a.bar + 1, a.group_blocks, a.err, kMsWaitNs);
       if (*(volatile int*)a.err) return;
       unsigned long long c = 0;
       if (threadIdx.x < S) c = __ldcg(&row[threadIdx.x]);
-      if (blockIdx.x == 0 && c) {  // only bits < k are ever counted
+      if (block == 0 && c) {  // only bits < k are ever counted
         reach += c;
         dsum += (unsigned long long)level * c;
         maxd = level;
@@ -449,7 +473,7 @@ __global__ void __launch_bounds__(kMsBlock) ms_persist_k(MsArgs a) {
         active.v[q] = ((unsigned long long)s_act[2 * q + 1] << 32) | s_act[2 * q];
       if (!mk_any(active)) break;
     }
-    if (blockIdx.x == 0 && threadIdx.x < k && a.reach) {
+    if (block == 0 && threadIdx.x < k && a.reach) {
       a.reach[s0 + threadIdx.x] = reach;
       a.dsum[s0 + threadIdx.x] = dsum;
       a.maxd[s0 + threadIdx.x] = maxd;
@@ -457,23 +481,37 @@ __global__ void __launch_bounds__(kMsBlock) ms_persist_k(MsArgs a) {
   }
 }
 
+// Groups and blocks per group for n nodes and a number of batches.
 template <int W>
-void ms_launch(MsArgs a, uint64_t n_sources, int device, cudaStream_t s) {
+void ms_shape(uint64_t n, uint64_t n_sources, int device, MsArgs& a) {
   int per_sm = 0;
-  UG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ms_persist_k<W>, kMsBlock, 0));
+  UG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ms_persist_k<W, true>, kMsBlock, 0));
   UG_CHECK(per_sm > 0, URSA_GPU_ECUDA, "msbfs: kernel cannot be resident");
-  // one warp per 32 nodes is all a level pass uses; fewer blocks make
-  // cheaper grid barriers
-  const uint64_t want = (a.n + 32 * kMsWarps - 1) / (32 * kMsWarps);
   const uint64_t cap = (uint64_t)per_sm * sm_count(device);
-  const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min(want, cap));
   const uint64_t batches = (n_sources + 64 * W - 1) / (64 * W);
-  const uint64_t per_launch = std::max<uint64_t>(1, kMsSourcesPerLaunch / (64 * W));
+  uint64_t groups = std::min(batches, cap * kMsNodesPerBlock / n);
+  groups = std::min({groups, kMsMaskBytes / (n * W * 32), kMsGroups});
+  groups = std::max<uint64_t>(1, groups);
+  const uint64_t rounds = (batches + groups - 1) / groups;  // as many groups as the rounds need
+  groups = (batches + rounds - 1) / rounds;
+  // one warp per 32 nodes is all a level pass uses; fewer blocks make
+  // cheaper barriers
+  const uint64_t want = (n + 32 * kMsWarps - 1) / (32 * kMsWarps);
+  a.groups = (uint32_t)groups;
+  a.group_blocks = (uint32_t)std::max<uint64_t>(1, std::min(want, cap / groups));
+}
+
+template <int W>
+void ms_launch(MsArgs a, uint64_t n_sources, cudaStream_t s) {
+  const uint64_t batches = (n_sources + 64 * W - 1) / (64 * W);
+  const uint64_t per_launch = std::max<uint64_t>(1, kMsSourcesPerLaunch / (64 * W)) * a.groups;
   for (uint64_t b = 0; b < batches; b += per_launch) {
     a.b_begin = b;
     a.b_end = std::min(batches, b + per_launch);
     void* args[] = {&a};
-    UG_CUDA(cudaLaunchCooperativeKernel((void*)ms_persist_k<W>, dim3(grid), dim3(kMsBlock), args, 0, s));
+    void* fn = a.groups > 1 ? (void*)ms_persist_k<W, true> : (void*)ms_persist_k<W, false>;
+    UG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(a.groups * a.group_blocks),
+                                        dim3(kMsBlock), args, 0, s));
     count_launch();
   }
 }
@@ -725,8 +763,7 @@ static const TopoImpl::MsHubs& ensure_ms_hubs(TopoImpl* t, int dir, const MsCsrs
 // Per source (device arrays of n_sources entries, or NULL): reach = nodes at
 // distance >= 1, dsum = their summed distances, maxd = eccentricity; d_dist
 // (or NULL): n_sources rows of n hop distances, -1 where unreached.
-// d_ctl: 4 zeroed words (grid barrier; word 2 turns nonzero if a barrier
-// wait expired).  Batches are 256 sources wide when there are enough
+// d_ctl: 4 zeroed words (word 2 turns nonzero if a barrier wait expired).  Batches are 256 sources wide when there are enough
 // sources to fill them and the masks of a graph of at most 2^21 nodes (64 MB
 // per mask array) stay in L2; otherwise 64 wide (fewer registers per
 // thread, more warps per SM).
@@ -738,14 +775,22 @@ static void msbfs_enqueue(TopoImpl* t, int dir, const uint32_t* d_src, uint64_t 
   const MsCsrs c = ms_csrs(t, dir, s);
   const TopoImpl::MsHubs& hb = ensure_ms_hubs(t, dir, c, s);
   const int W = n_sources >= 256 && n <= (1ull << 21) ? 4 : 1;
-  Scratch<unsigned long long> visited(n * W, s), fa(n * W, s), fb(n * W, s), acc(n * W, s);
-  Scratch<unsigned long long> count(3 * (64 * W + 8), s);
-  UG_CUDA(cudaMemsetAsync(acc.get(), 0, n * W * 8, s));
-  const uint64_t nh = hb.n_hubs, nc = hb.n_chunks;
-  Scratch<unsigned long long> hacc((nh ? nh : 1) * W, s);
-  UG_CUDA(cudaMemsetAsync(hacc.get(), 0, (nh ? nh : 1) * W * 8, s));
-  if (d_dist) UG_CUDA(cudaMemsetAsync(d_dist, 0xFF, n_sources * n * 4, s));
   MsArgs a;
+  if (W == 4)
+    ms_shape<4>(n, n_sources, t->device, a);
+  else
+    ms_shape<1>(n, n_sources, t->device, a);
+  const uint64_t words = a.groups * n * W;
+  Scratch<unsigned long long> visited(words, s), fa(words, s), fb(words, s), acc(words, s);
+  Scratch<unsigned long long> count(a.groups * 3 * (64 * W + 8), s);
+  Scratch<unsigned> bar(a.groups * 2, s);
+  UG_CUDA(cudaMemsetAsync(acc.get(), 0, words * 8, s));
+  UG_CUDA(cudaMemsetAsync(bar.get(), 0, a.groups * 2 * sizeof(unsigned), s));
+  const uint64_t nh = hb.n_hubs, nc = hb.n_chunks;
+  const uint64_t hub_words = a.groups * (nh ? nh : 1) * W;
+  Scratch<unsigned long long> hacc(hub_words, s);
+  UG_CUDA(cudaMemsetAsync(hacc.get(), 0, hub_words * 8, s));
+  if (d_dist) UG_CUDA(cudaMemsetAsync(d_dist, 0xFF, n_sources * n * 4, s));
   a.in_off = c.pull_off;
   a.in_src = c.pull_src;
   a.out_off = c.push_off;
@@ -769,12 +814,12 @@ static void msbfs_enqueue(TopoImpl* t, int dir, const uint32_t* d_src, uint64_t 
   a.reach = d_reach;
   a.dsum = d_dsum;
   a.maxd = d_maxd;
-  a.bar = d_ctl;
+  a.bar = bar.get();
   a.err = (int*)(d_ctl + 2);
   if (W == 4)
-    ms_launch<4>(a, n_sources, t->device, s);
+    ms_launch<4>(a, n_sources, s);
   else
-    ms_launch<1>(a, n_sources, t->device, s);
+    ms_launch<1>(a, n_sources, s);
 }
 
 // Hop distances from each of the device ids d_src (< n), following `dir`:
