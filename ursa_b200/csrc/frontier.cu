@@ -1,9 +1,6 @@
 // frontier.cu -- BFS family on the device (ursa-core/src/algo/bfs.rs, hop.rs).
 //
-//  * bfs_distances: level-synchronous, direction-optimising (top-down frontier
-//    queue while the frontier's edges are few, bottom-up over unvisited nodes
-//    when they are many, Beamer et al.); levels are exact, so the output is
-//    bit-identical to the reference's serial BFS.
+//  * bfs_distances: bfs.cu.
 //  * k_hop / shortest_path: exact-order expansion.  The reference walks the
 //    frontier in order and each node's neighbours in CSR order, and the first
 //    walk that reaches v discovers it (hop.rs:106-123, bfs.rs:69-87).  Here
@@ -121,77 +118,6 @@ __global__ void unmark_k(const uint32_t* __restrict__ N, uint64_t cnt, uint8_t* 
 
 __global__ void set_one_u8_k(uint8_t* p, uint64_t i, uint8_t v) { p[i] = v; }
 __global__ void set_one_u32_k(uint32_t* p, uint64_t i, uint32_t v) { p[i] = v; }
-__global__ void set_one_i32_k(int32_t* p, uint64_t i, int32_t v) { p[i] = v; }
-__global__ void fill_u32_k(uint32_t* p, uint64_t n, uint32_t v) {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (uint64_t)gridDim.x * blockDim.x)
-    p[i] = v;
-}
-
-// Warp-aggregated append of v to Q (count at *cnt).
-__device__ __forceinline__ void append(uint32_t* Q, uint32_t* cnt, bool take, uint32_t v) {
-  uint32_t mask = __ballot_sync(__activemask(), take);
-  if (!take) return;
-  int lane = threadIdx.x & 31;
-  int leader = __ffs(mask) - 1;
-  uint32_t base = 0;
-  if (lane == leader) base = atomicAdd(cnt, (uint32_t)__popc(mask));
-  base = __shfl_sync(mask, base, leader);
-  Q[base + __popc(mask & ((1u << lane) - 1u))] = v;
-}
-
-// Adds, per warp, the forward degrees of the nodes this round appended to the
-// next frontier (the next level's scout count, read with the frontier size).
-__device__ __forceinline__ void add_scout(DirView fwd, bool take, uint32_t v,
-                                          unsigned long long* __restrict__ scout) {
-  unsigned long long x = take ? (unsigned long long)dv_deg(fwd, v) : 0ull;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-  if ((threadIdx.x & 31) == 0 && x) atomicAdd(scout, x);
-}
-
-__global__ void td_k(DirView d, const uint32_t* __restrict__ F, uint64_t f,
-                     const uint64_t* __restrict__ pos, uint64_t T, int32_t* dist, int32_t level,
-                     uint32_t* __restrict__ N, uint32_t* __restrict__ cnt,
-                     unsigned long long* __restrict__ scout) {
-  uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  uint64_t span = ((T + stride - 1) / stride) * stride;  // whole warps iterate together
-  for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < span; e += stride) {
-    bool take = false;
-    uint32_t v = 0;
-    if (e < T) {
-      uint64_t i = owner_in_pos(pos, f, e);
-      v = dv_nbr(d, F[i], (uint32_t)(e - pos[i]));
-      if (dist[v] < 0) take = atomicCAS(&dist[v], -1, level + 1) == -1;
-    }
-    append(N, cnt, take, v);
-    add_scout(d, take, v, scout);
-  }
-}
-
-__global__ void bu_k(DirView rev, DirView fwd, uint64_t n, int32_t* dist, int32_t level,
-                     uint32_t* __restrict__ N, uint32_t* __restrict__ cnt,
-                     unsigned long long* __restrict__ scout) {
-  uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  uint64_t span = ((n + stride - 1) / stride) * stride;
-  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < span; v += stride) {
-    bool take = false;
-    if (v < n && dist[v] < 0) {
-      uint32_t deg = dv_deg(rev, (uint32_t)v);
-      for (uint32_t j = 0; j < deg; j++) {
-        uint32_t u = dv_nbr(rev, (uint32_t)v, j);
-        if (dist[u] == level) {
-          dist[v] = level + 1;
-          take = true;
-          break;
-        }
-      }
-    }
-    append(N, cnt, take, (uint32_t)v);
-    add_scout(fwd, take, (uint32_t)v, scout);
-  }
-}
-
 // Walk parents from target back to source into path (reversed at the end).
 __global__ void backtrack_k(const uint32_t* __restrict__ parent, uint32_t source, uint32_t target,
                             uint64_t cap, uint32_t* __restrict__ path, uint64_t* __restrict__ len) {
@@ -208,12 +134,6 @@ __global__ void backtrack_k(const uint32_t* __restrict__ parent, uint32_t source
     path[l - 1 - i] = x;
   }
   *len = l;
-}
-
-__global__ void fill_seed_k(uint32_t* p, uint64_t n, uint32_t v) {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (uint64_t)gridDim.x * blockDim.x)
-    p[i] = v;
 }
 
 }  // namespace
@@ -276,69 +196,6 @@ uint32_t expand_exact(const DirView& d, uint64_t n, const uint32_t* F, uint32_t 
     UG_LAUNCH_CHECK();
   }
   return cnt;
-}
-
-// ------------------------------------------------------------- bfs_distances
-void bfs_distances_run(TopoImpl* t, uint32_t source, int dir, int32_t* d_dist, cudaStream_t s) {
-  const uint64_t n = t->n;
-  if (n == 0) return;
-  UG_CUDA(cudaMemsetAsync(d_dist, 0xFF, n * sizeof(int32_t), s));
-  if ((uint64_t)source >= n) return;  // bfs.rs:21-23
-  DirView fw = dir_view(t, dir, s);
-  DirView rv = reverse_view(t, dir, s);
-  FrontierBufs b;
-  b.alloc(n, s);
-  set_one_i32_k<<<1, 1, 0, s>>>(d_dist, source, 0);
-  UG_LAUNCH_CHECK();
-  set_one_u32_k<<<1, 1, 0, s>>>(b.F.get(), 0, source);
-  UG_LAUNCH_CHECK();
-  uint32_t f = 1;
-  int32_t level = 0;
-  bool bottom_up = false;
-  const double total_edges = (double)t->m * (dir == 2 ? 2.0 : 1.0);
-  double edges_left = total_edges;
-  const double alpha = 14.0, beta = 24.0;
-  // the frontier's out-edge total ("scout count"): the source's degree, then
-  // summed on the device by each level's kernel as it appends the next
-  // frontier, so a level costs one host read (frontier size and scout count)
-  Scratch<unsigned long long> scout(1, s);
-  uint64_t T = frontier_scan(fw, b.F.get(), f, b.pos.get(), s);
-  while (f > 0) {
-    UG_CUDA(cudaMemsetAsync(b.count.get(), 0, sizeof(uint32_t), s));
-    UG_CUDA(cudaMemsetAsync(scout.get(), 0, sizeof(unsigned long long), s));
-    if (!bottom_up) {
-      if ((double)T > edges_left / alpha) {
-        bottom_up = true;
-      } else {
-        if (T) {
-          // edge-balanced expansion: the frontier's degree prefix (its total is T)
-          fdeg_k<<<grid_for((uint64_t)f + 1), kBlock, 0, s>>>(fw, b.F.get(), f, b.pos.get());
-          UG_LAUNCH_CHECK();
-          exclusive_scan_u64(b.pos.get(), b.pos.get(), (uint64_t)f + 1, nullptr, s);
-          td_k<<<grid_for(T, kBlock, 148u * 64u), kBlock, 0, s>>>(fw, b.F.get(), f, b.pos.get(), T,
-                                                                   d_dist, level, b.N.get(),
-                                                                   b.count.get(), scout.get());
-          UG_LAUNCH_CHECK();
-        }
-        edges_left -= (double)T;
-      }
-    }
-    if (bottom_up) {
-      bu_k<<<grid_for(n, kBlock, 148u * 64u), kBlock, 0, s>>>(rv, fw, n, d_dist, level, b.N.get(),
-                                                               b.count.get(), scout.get());
-      UG_LAUNCH_CHECK();
-    }
-    uint32_t next = 0;
-    unsigned long long t_next = 0;
-    UG_CUDA(cudaMemcpyAsync(&next, b.count.get(), sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    UG_CUDA(cudaMemcpyAsync(&t_next, scout.get(), sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-    UG_CUDA(cudaStreamSynchronize(s));
-    if (bottom_up && (double)next < (double)n / beta && next < f) bottom_up = false;
-    swap(b.F, b.N);
-    f = next;
-    T = t_next;
-    level++;
-  }
 }
 
 // ------------------------------------------------------------------- k_hop
@@ -456,21 +313,6 @@ struct ursa_gpu_pairs {
 using namespace ug;
 
 extern "C" {
-
-int ursa_gpu_bfs_distances(ursa_gpu_topo* t, uint32_t source, int dir, int32_t* out) {
-  return guard([&] {
-    UG_CHECK(t, URSA_GPU_EINVAL, "topology is NULL");
-    UG_CHECK(dir >= 0 && dir <= 2, URSA_GPU_EINVAL, "direction must be 0, 1 or 2");
-    TopoImpl* ti = &t->impl;
-    if (ti->n == 0) return;
-    UG_CHECK(out, URSA_GPU_EINVAL, "out is NULL");
-    cudaStream_t s = thread_stream(ti->device);
-    Scratch<int32_t> d(ti->n, s);
-    bfs_distances_run(ti, source, dir, d.get(), s);
-    UG_CUDA(cudaMemcpyAsync(out, d.get(), ti->n * 4, cudaMemcpyDeviceToHost, s));
-    UG_CUDA(cudaStreamSynchronize(s));
-  });
-}
 
 int ursa_gpu_shortest_path(ursa_gpu_topo* t, uint32_t source, uint32_t target, int dir,
                            uint32_t* path, uint64_t cap, int64_t* len) {
