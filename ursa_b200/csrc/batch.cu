@@ -33,6 +33,7 @@
 #include <cstring>
 #include <vector>
 
+#include "tcstream.cuh"
 #include "frontier.cuh"
 #include "primitives.cuh"
 #include "batch.cuh"
@@ -135,30 +136,58 @@ struct PrIter {
   u128 delta, dang;
 };
 
-template <int G>
-__device__ __forceinline__ void bk_class_unit(const GraphDesc& g, uint32_t lo, uint32_t hi,
-                                              uint32_t unit, PrIter& it) {
-  const int lane = threadIdx.x & 31;
-  const int sub = lane % G;
-  const uint32_t idx = lo + unit * (32u / G) + (uint32_t)(lane / G);
-  const bool valid = idx < hi;
-  uint32_t r = 0, b = 0, e = 0;
-  if (valid) {
-    r = g.rows[idx];
-    b = g.in_off[r];
-    e = g.in_off[r + 1];
+// A warp's unit of rows: the lane's row and what its update needs, loaded one
+// unit ahead (row, then the rest): with one CTA per SM a unit alone is a chain
+// of five dependent loads.
+struct BkUnit {
+  int c;         // class: 32 >> c lanes per row
+  uint32_t idx;  // the lane's place in the class order, `none` past the class's end
+  uint32_t r, b, e, od;
+  double old;
+};
+constexpr uint32_t kBkNone = 0xFFFFFFFFu;
+
+__device__ __forceinline__ BkUnit bk_unit_row(const GraphDesc& g, const BkShared& sh, uint32_t u) {
+  BkUnit x;
+  x.c = 0;
+  x.idx = kBkNone;
+  x.r = 0;
+  if (u >= sh.unit_begin[6]) return x;
+#pragma unroll
+  for (int k = 1; k < 6; k++)
+    if (u >= sh.unit_begin[k]) x.c = k;
+  const uint32_t idx = g.cls[x.c] + ((u - sh.unit_begin[x.c]) << x.c) + ((threadIdx.x & 31) >> (5 - x.c));
+  if (idx < g.cls[x.c + 1]) {
+    x.idx = idx;
+    x.r = g.rows[idx];
   }
-  F2 acc = bk_row_sum<G, (G >= 32 ? 8 : 4)>(g.in_src, it.xr, g.id_base, b, e, sub);
+  return x;
+}
+
+__device__ __forceinline__ void bk_unit_load(const GraphDesc& g, BkUnit& x) {
+  x.b = x.e = x.od = 0;
+  x.old = 0.0;
+  if (x.idx == kBkNone) return;
+  x.b = g.in_off[x.r];
+  x.e = g.in_off[x.r + 1];
+  if (((threadIdx.x & 31) & ((32u >> x.c) - 1)) == 0) {  // the lane that finishes the row
+    x.old = g.rank[x.r];
+    x.od = g.out_off[x.r + 1] - g.out_off[x.r];
+  }
+}
+
+template <int G>
+__device__ __forceinline__ void bk_class_unit(const GraphDesc& g, const BkUnit& x, PrIter& it) {
+  const int sub = (threadIdx.x & 31) % G;
+  F2 acc = bk_row_sum<G, (G >= 32 ? 8 : 4)>(g.in_src, it.xr, g.id_base, x.b, x.e, sub);
   acc = bk_group_sum<G>(acc);
-  if (valid && sub == 0) {
+  if (x.idx != kBkNone && sub == 0) {
     // next[u] = base + d * contrib(u)   (pagerank.rs:81-83)
-    const double old = g.rank[r];
     const double nx = __dadd_rn(it.base, __dmul_rn(it.damping, f2_value(acc)));
-    it.delta += fx_of(fabs(__dsub_rn(nx, old)));
-    g.rank[r] = nx;
-    const uint32_t od = g.out_off[r + 1] - g.out_off[r];
-    it.xw[r] = od ? __double2float_rn(__ddiv_rn(nx, (double)od)) : 0.f;
-    if (!od) it.dang += fx_of(nx);
+    it.delta += fx_of(fabs(__dsub_rn(nx, x.old)));
+    g.rank[x.r] = nx;
+    it.xw[x.r] = x.od ? __double2float_rn(__ddiv_rn(nx, (double)x.od)) : 0.f;
+    if (!x.od) it.dang += fx_of(nx);
   }
 }
 
@@ -206,20 +235,21 @@ __device__ void bk_pagerank(const BucketArgs& A, BkShared& sh, float* sx, uint32
     it.damping = A.damping;
     it.delta = 0;
     it.dang = 0;
+    BkUnit next = bk_unit_row(g, sh, warp);
+    bk_unit_load(g, next);
+    BkUnit after = bk_unit_row(g, sh, warp + NT / 32);
     for (uint32_t u = warp; u < n_units; u += NT / 32) {
-      int c = 0;
-#pragma unroll
-      for (int k = 1; k < 6; k++)
-        if (u >= sh.unit_begin[k]) c = k;
-      const uint32_t unit = u - sh.unit_begin[c];
-      const uint32_t lo = g.cls[c], hi = g.cls[c + 1];
-      switch (c) {
-        case 0: bk_class_unit<32>(g, lo, hi, unit, it); break;
-        case 1: bk_class_unit<16>(g, lo, hi, unit, it); break;
-        case 2: bk_class_unit<8>(g, lo, hi, unit, it); break;
-        case 3: bk_class_unit<4>(g, lo, hi, unit, it); break;
-        case 4: bk_class_unit<2>(g, lo, hi, unit, it); break;
-        default: bk_class_unit<1>(g, lo, hi, unit, it); break;
+      const BkUnit x = next;
+      next = after;
+      bk_unit_load(g, next);
+      after = bk_unit_row(g, sh, u + 2 * (NT / 32));
+      switch (x.c) {
+        case 0: bk_class_unit<32>(g, x, it); break;
+        case 1: bk_class_unit<16>(g, x, it); break;
+        case 2: bk_class_unit<8>(g, x, it); break;
+        case 3: bk_class_unit<4>(g, x, it); break;
+        case 4: bk_class_unit<2>(g, x, it); break;
+        default: bk_class_unit<1>(g, x, it); break;
       }
     }
     block_sum2<NT>(it.delta, it.dang, sh, delta, dm);
@@ -257,18 +287,32 @@ __device__ void bk_components(BkShared& sh, uint32_t* par) {
   const uint32_t n = g.n;
   for (uint32_t u = threadIdx.x; u < n; u += NT) par[u] = u;
   __syncthreads();
+  // slots in spans of four per thread; warp 0 finds the rows that own a span's
+  // first and last slot by searching forward from the last span's (a search
+  // over all rows per 1,024 edges by one thread was most of the time)
   const uint32_t ob = g.o_off[0], oe = g.o_off[n];
-  for (uint32_t base = ob; base < oe; base += NT) {
-    if (threadIdx.x == 0) {
-      const uint32_t last = base + NT - 1 < oe ? base + NT - 1 : oe - 1;
-      sh.range[0] = owner_of(g.o_off, n, base);
-      sh.range[1] = owner_of(g.o_off, n, last);
+  constexpr uint32_t kSpan = 4 * NT;
+  uint32_t prev = 0;
+  for (uint32_t base = ob; base < oe; base += kSpan) {
+    const uint32_t last = min(base + kSpan, oe) - 1;
+    if (threadIdx.x < 32) {
+      const uint32_t lo = warp_owner_from(g.o_off, n, prev, base);
+      prev = warp_owner_from(g.o_off, n, lo, last);
+      if (threadIdx.x == 0) {
+        sh.range[0] = lo;
+        sh.range[1] = prev;
+      }
     }
     __syncthreads();
-    const uint32_t k = base + threadIdx.x;
-    if (k < oe) {
-      const uint32_t u = bk_owner_between(g.o_off, sh.range[0], sh.range[1], k);
-      uf_unite(par, u, g.o_tgt[k] - g.id_base);
+#pragma unroll
+    for (uint32_t q = 0; q < 4; q++) {
+      const uint32_t k = base + q * NT + threadIdx.x;
+      if (k <= last) {
+        const uint32_t u = bk_owner_between(g.o_off, sh.range[0], sh.range[1], k);
+        const uint32_t v = g.o_tgt[k] - g.id_base;
+        // most edges join what has a common parent by now
+        if (uf_parent(par, u) != uf_parent(par, v)) uf_unite(par, u, v);
+      }
     }
     __syncthreads();
   }
@@ -286,9 +330,12 @@ __device__ void bk_components(BkShared& sh, uint32_t* par) {
 // concatenation, located by a warp scan of the list lengths -- and every w
 // found in the bitmap closes the triangle {u, v, w}, counted once (u < v < w
 // in the orientation's rank order) and credited to all three vertices: u's
-// credit once per vertex, v's once per run of lanes on the same v, w's per
-// hit.  A 32-element chunk inside one or two lists (the common case) needs
-// no per-lane search.  Graphs above kTcBitCap nodes use a per-lane sorted merge.
+// and v's credit once per list (the counts of tc_stream), w's per hit.  Graphs
+// above kTcBitCap nodes use a per-lane sorted merge.  Bound by issue (0.58 of a
+// slot per scheduler and cycle, 65 instructions per 32 probes) and by how
+// unevenly the units weigh: 1,000 graphs 9.65 ms before the shared probe loop
+// with the next elements in flight, 8.0 now; units of 8 or 16 vertices pay
+// more in grabs than they balance (11.2, 9.0 ms), dealing them out is worse.
 constexpr uint32_t kTcBitCap = 65536;  // nodes per graph on the bitmap path
 
 struct TcArgs {
@@ -305,6 +352,7 @@ __global__ void __launch_bounds__(NT) tc_batch_k(TcArgs A) {
   extern __shared__ __align__(16) uint32_t tc_smem[];
   const uint32_t FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
+  __shared__ uint32_t pack[NT / 32][32];
   uint32_t* bm = tc_smem + (threadIdx.x >> 5) * A.words;
   // every vertex clears the bits it sets, so the bitmap is zeroed once
   for (uint32_t i = lane; i < A.words; i += 32) bm[i] = 0u;
@@ -322,9 +370,13 @@ __global__ void __launch_bounds__(NT) tc_batch_k(TcArgs A) {
     const uint32_t n = gd->n, idb = gd->id_base;
     const uint32_t last = un.y + A.unit_len < n ? un.y + A.unit_len : n;
     const bool bitmap = n <= A.words * 32u;
-    for (uint32_t u = un.y; u < last; u++) {
-      const uint32_t ob = off[u], oe = off[u + 1];
-      if (oe - ob < 2) continue;  // u is the lowest vertex of no triangle
+    for (uint32_t u0 = un.y; u0 < last; u0 += 32)  // 32 rows' offsets at a time
+    for (uint32_t rb = u0 + lane < last ? off[u0 + lane] : 0u,
+                  re = u0 + lane < last ? off[u0 + lane + 1] : 0u,
+                  todo = __ballot_sync(FULL, re - rb >= 2);  // else the lowest vertex of no triangle
+         todo; todo &= todo - 1) {
+      const uint32_t from_lane = __ffs(todo) - 1, u = u0 + from_lane;
+      const uint32_t ob = __shfl_sync(FULL, rb, from_lane), oe = __shfl_sync(FULL, re, from_lane);
       uint32_t cu = 0;
       if (bitmap) {
         for (uint32_t i = ob + lane; i < oe; i += 32) {
@@ -340,55 +392,19 @@ __global__ void __launch_bounds__(NT) tc_batch_k(TcArgs A) {
             st = off[v];
             len = off[v + 1] - st;
           }
-          uint32_t incl = len;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(FULL, incl, o);
-            if (lane >= o) incl += t;
-          }
-          const uint32_t total = __shfl_sync(FULL, incl, 31);
-          const uint32_t excl = incl - len;
-          const uint32_t nonempty = __ballot_sync(FULL, len > 0);
-          for (uint32_t pb = 0; pb < total; pb += 32) {
-            const uint32_t p = pb + lane;
-            const uint32_t lim = pb + 32 < total ? pb + 32 : total;
-            // first list still live at pb (non-empty: its end exceeds pb)
-            const uint32_t j0 = __popc(__ballot_sync(FULL, incl <= pb));
-            const uint32_t end0 = __shfl_sync(FULL, incl, j0);
-            const bool one_list = end0 >= lim;
-            uint32_t j = j0;
-            if (!one_list) {
-              const uint32_t after = j0 < 31 ? nonempty & (0xfffffffeu << j0) : 0u;
-              const uint32_t j1 = after ? (uint32_t)(__ffs(after) - 1) : 31u;
-              if (__shfl_sync(FULL, incl, j1) >= lim) {
-                j = p < end0 ? j0 : j1;  // the chunk spans two lists
-              } else {
-                j = 0;  // first lane whose inclusive end exceeds p
-#pragma unroll
-                for (int step = 16; step >= 1; step >>= 1) {
-                  const uint32_t t = __shfl_sync(FULL, incl, j + step - 1);
-                  if (t <= p) j += step;
-                }
-              }
-            }
-            const uint32_t vj = __shfl_sync(FULL, v, j);
-            const uint32_t sj = __shfl_sync(FULL, st, j);
-            const uint32_t ej = __shfl_sync(FULL, excl, j);
+          uint32_t from;
+          const uint32_t c = tc_stream<true>(pack[threadIdx.x >> 5], st, len, tgt, &from, [&](uint32_t, uint32_t w) {
             bool hit = false;
-            if (p < total) {
-              const uint32_t w = tgt[sj + (p - ej)] - idb;
+            if (w != kTcEmpty) {
+              w -= idb;
               hit = (bm[w >> 5] >> (w & 31)) & 1u;
               if (hit) atomicAdd(&tri[w], 1u);
             }
-            const uint32_t hits = __ballot_sync(FULL, hit);
-            if (hits) {
-              cu += hit ? 1u : 0u;
-              // v's credit: one atomic per run of lanes on the same v
-              const uint32_t run = one_list ? FULL : __match_any_sync(FULL, j);
-              const uint32_t c = __popc(run & hits);
-              if (c && lane == __ffs(run) - 1) atomicAdd(&tri[vj], c);
-            }
-          }
+            return hit;
+          });
+          v = __shfl_sync(FULL, v, from);
+          if (c) atomicAdd(&tri[v], c);
+          cu += c;
         }
         __syncwarp();
         for (uint32_t i = ob + lane; i < oe; i += 32) bm[(tgt[i] - idb) >> 5] = 0u;

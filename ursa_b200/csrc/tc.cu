@@ -16,6 +16,7 @@
 // hash slot, flushed once per v).  Integer results are order-independent, so
 // the counts are bit-identical to the reference.
 #include "frontier.cuh"
+#include "tcstream.cuh"
 
 namespace ug {
 
@@ -48,7 +49,6 @@ __global__ void orient_fill_k(const uint32_t* __restrict__ off, const uint32_t* 
 }
 
 constexpr uint32_t kTcGrab = 16;
-constexpr uint32_t kTcEmpty = 0xFFFFFFFFu;
 
 __device__ __forceinline__ uint32_t tc_hash(uint32_t w, uint32_t bits) {
   return (w * 0x9E3779B1u) >> (32 - bits);
@@ -137,67 +137,6 @@ __device__ __forceinline__ void tc_table_flush(uint32_t* T, uint32_t* C, uint32_
   }
 }
 
-// Streams up to 32 (u, v) pairs' suffixes back to back through a warp: lane l
-// takes probe pb + l of the concatenation; hit(j, w) is called by every lane
-// with the pair's lane j and the element (kTcEmpty without a probe) and says
-// whether it closes a triangle.  Lane k holds pair k: the first slot b and the
-// length len of its suffix (0: no pair).  The pairs with probes are first
-// moved to the front, so that each owns at least one probe and a round finds
-// its pairs with one ballot and one OR of the ends inside the round, in place
-// of a five-step shuffle search; and each lane counts the hits of the pair
-// that moved to it from the ballot of the round's hits, in place of a
-// shared-memory atomic per hit.  Returns that count, and the lane the pair
-// came from in *from_lane.
-template <class F>
-__device__ __forceinline__ uint32_t tc_stream(uint32_t* pack, uint32_t b, uint32_t len,
-                                              const uint32_t* __restrict__ tgt,
-                                              uint32_t* from_lane, F&& hit) {
-  const uint32_t FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  const uint32_t lt = (1u << lane) - 1u;
-  const uint32_t some = __ballot_sync(FULL, len != 0);
-  const int count = __popc(some);
-  if (len) pack[__popc(some & lt)] = lane;
-  __syncwarp();
-  const uint32_t from = lane < count ? pack[lane] : 0u;
-  __syncwarp();
-  *from_lane = from;
-  b = __shfl_sync(FULL, b, from);
-  len = __shfl_sync(FULL, len, from);
-  if (lane >= count) len = 0;
-  uint32_t incl = len;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(FULL, incl, o);
-    if (lane >= o) incl += t;
-  }
-  const uint32_t total = __shfl_sync(FULL, incl, 31);
-  const uint32_t excl = incl - len;
-  const uint32_t start = b - excl;  // probe p of pair k is tgt[start_k + p]
-  uint32_t c = 0;
-  for (uint32_t pb = 0; pb < total; pb += 32) {
-    // pairs that end at or before pb, and those that end inside the round:
-    // one that ends after `at` probes leaves the lanes from `at` to the next
-    const uint32_t first = __popc(__ballot_sync(FULL, lane < count && incl <= pb));
-    const uint32_t at = incl - pb;
-    const bool inside = lane < count && incl > pb && at < 32;
-    const uint32_t ends = __reduce_or_sync(FULL, inside ? 1u << (at & 31) : 0u);
-    const uint32_t k = first + __popc(ends & (lt | (1u << lane)));
-    const uint32_t sk = __shfl_sync(FULL, start, k & 31);
-    const uint32_t j = __shfl_sync(FULL, from, k & 31);
-    const uint32_t p = pb + lane;
-    const bool h = hit(j, p < total ? tgt[sk + p] : kTcEmpty);
-    __syncwarp();
-    const uint32_t hits = __ballot_sync(FULL, h);
-    if (len && incl > pb && excl < pb + 32) {  // this lane's pair is in the round
-      const uint32_t lo = excl > pb ? excl - pb : 0u;
-      const uint32_t upto = at < 32 ? (1u << at) - 1u : FULL;
-      c += __popc(hits & upto & ~((1u << lo) - 1u));
-    }
-  }
-  return c;
-}
-
 // One warp: `group` (at most 32) entries of [i0, ie) at a time, `stride`
 // apart; credits each u and returns the warp's hit count (all lanes).
 __device__ __forceinline__ uint32_t tc_pairs(uint32_t* T, uint32_t* C, uint32_t* pack, uint32_t bits,
@@ -219,7 +158,7 @@ __device__ __forceinline__ uint32_t tc_pairs(uint32_t* T, uint32_t* C, uint32_t*
       len = off[u + 1] - b;
     }
     uint32_t from;
-    const uint32_t c = tc_stream(pack, b, len, tgt, &from, [&](uint32_t, uint32_t w) {
+    const uint32_t c = tc_stream<false>(pack, b, len, tgt, &from, [&](uint32_t, uint32_t w) {
       const uint32_t h = tc_find(T, bits, w);
       if (h != kTcEmpty) atomicAdd(&C[h], 1u);
       return h != kTcEmpty;
@@ -316,7 +255,7 @@ __global__ void __launch_bounds__(256) tc_middle_search_k(TcArgs a) {
       }
       if (!__any_sync(FULL, len != 0)) continue;
       uint32_t from;
-      const uint32_t c = tc_stream(pack[wid], b, len, a.tgt, &from, [&](uint32_t j, uint32_t w) {
+      const uint32_t c = tc_stream<true>(pack[wid], b, len, a.tgt, &from, [&](uint32_t j, uint32_t w) {
         uint32_t lo = __shfl_sync(FULL, ob, j);
         uint32_t left = __shfl_sync(FULL, dv, j);
         if (w == kTcEmpty) left = 0;
@@ -450,10 +389,8 @@ __global__ void __launch_bounds__(kWarps * 32) tc_middle_block_k(TcArgs a, uint3
 // orientation counts instead: a warp per vertex u puts N+(u) in a
 // shared-memory hash set (open addressing, load <= 1/2; longer lists are
 // searched by binary search in global memory) and streams the concatenation
-// of N+(v), v in N+(u), 32 lists at a time with lane p taking element p (its
-// list found by a warp scan of the lengths and a shuffle binary search); a
-// hit w is the triangle (u, v, w), credited to w at once and to v and u
-// through per-list counters in shared memory.
+// of N+(v), v in N+(u), 32 lists at a time; a hit w is the triangle (u, v, w),
+// credited to w at once and to v and u by the lists' counts.
 constexpr uint64_t kSmallEntries = 1u << 18;
 constexpr int kSmThreads = 256;
 constexpr int kSmWarps = kSmThreads / 32;
@@ -468,9 +405,8 @@ __global__ void __launch_bounds__(kSmThreads) count_small_k(const uint32_t* __re
   const uint32_t FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   uint32_t* T = tc_sm + (size_t)w * kSmSlots;
-  uint32_t* cnt = tc_sm + (size_t)kSmWarps * kSmSlots + w * 32;
+  uint32_t* pack = tc_sm + (size_t)kSmWarps * kSmSlots + w * 32;
   for (uint32_t i = lane; i < kSmSlots; i += 32) T[i] = kTcEmpty;
-  cnt[lane] = 0;
   __syncwarp();
   while (true) {
     unsigned long long g = 0;
@@ -502,60 +438,33 @@ __global__ void __launch_bounds__(kSmThreads) count_small_k(const uint32_t* __re
           st = o_off[v];
           len = o_off[v + 1] - st;
         }
-        uint32_t incl = len;  // inclusive scan of the list lengths
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const uint32_t t = __shfl_up_sync(FULL, incl, o);
-          if (lane >= o) incl += t;
-        }
-        const uint32_t total = __shfl_sync(FULL, incl, 31);
-        for (uint32_t pb = 0; pb < total; pb += 32) {
-          const uint32_t p = pb + lane;
-          uint32_t j = 0;  // first list whose inclusive end exceeds p
-#pragma unroll
-          for (int step = 16; step >= 1; step >>= 1) {
-            const uint32_t t = __shfl_sync(FULL, incl, j + step - 1);
-            if (t <= p) j += step;
-          }
-          const uint32_t sj = __shfl_sync(FULL, st, j & 31);
-          const uint32_t ij = __shfl_sync(FULL, incl, j & 31);
-          const uint32_t lj = __shfl_sync(FULL, len, j & 31);
-          if (p < total) {
-            const uint32_t x = o_tgt[sj + (p - (ij - lj))];
-            bool hit = false;
-            if (hashed) {
-              uint32_t h = tc_hash(x, bits);
-              while (true) {
-                const uint32_t t = T[h];
-                if (t == x) {
-                  hit = true;
-                  break;
-                }
-                if (t == kTcEmpty) break;
-                h = (h + 1) & mask;
-              }
-            } else {
-              uint32_t lo = ob, hi = oe;
-              while (lo < hi) {
-                const uint32_t mid = (lo + hi) >> 1;
-                if (o_tgt[mid] < x) lo = mid + 1; else hi = mid;
-              }
-              hit = lo < oe && o_tgt[lo] == x;
+        uint32_t from;
+        const uint32_t c = tc_stream<true>(pack, st, len, o_tgt, &from, [&](uint32_t, uint32_t x) {
+          bool hit = false;
+          if (hashed) {  // the warp steps together until its last lane is done
+            uint32_t h = tc_hash(x, bits);
+            bool open = x != kTcEmpty;
+            do {
+              const uint32_t t = T[h];
+              hit |= open && t == x;
+              open = open && t != x && t != kTcEmpty;
+              h = (h + 1) & mask;
+            } while (__any_sync(FULL, open));
+          } else if (x != kTcEmpty) {
+            uint32_t lo = ob, left = oe - ob;
+            while (left > 1) {  // the last element <= x, or the first one
+              const uint32_t half = left >> 1;
+              if (o_tgt[lo + half] <= x) lo += half;
+              left -= half;
             }
-            if (hit) {
-              atomicAdd(&tri[x], 1u);
-              atomicAdd(&cnt[j], 1u);
-            }
+            hit = o_tgt[lo] == x;
           }
-        }
-        __syncwarp();
-        const uint32_t c = cnt[lane];
-        if (c) {
-          atomicAdd(&tri[v], c);
-          cu += c;
-          cnt[lane] = 0;
-        }
-        __syncwarp();
+          if (hit) atomicAdd(&tri[x], 1u);
+          return hit;
+        });
+        v = __shfl_sync(FULL, v, from);
+        if (c) atomicAdd(&tri[v], c);
+        cu += c;
       }
       cu = __reduce_add_sync(FULL, cu);
       if (lane == 0 && cu) atomicAdd(&tri[u], cu);
