@@ -31,8 +31,8 @@
 
 namespace ug {
 
-void sssp_run(const DirView& d, const double* w0, const double* w1, uint64_t n, uint32_t source,
-              unsigned long long* dist, cudaStream_t s);
+void sssp_run(const DirView& d, const double* w0, const double* w1, uint64_t n, uint64_t m,
+              uint32_t source, unsigned long long* dist, cudaStream_t s);
 
 namespace {
 
@@ -1178,7 +1178,7 @@ static void brandes_source(TopoImpl* t, const double* w_out, uint32_t src, BcSta
     dv.off0 = off;
     dv.tgt0 = tgt;
     dv.eid0 = t->out.eid.get();
-    sssp_run(dv, w_out, nullptr, n, src, st.dist.get(), s);
+    sssp_run(dv, w_out, nullptr, n, m, src, st.dist.get(), s);
     UG_CUDA(cudaMemsetAsync(st.indeg.get(), 0, n * 4, s));
     if (m) {
       tight_indeg_k<<<grid_for(m, kBlock, 148u * 64u), kBlock, 0, s>>>(off, tgt, w_out, n, m,

@@ -25,8 +25,6 @@ namespace ug {
 
 namespace {
 
-constexpr uint32_t kSpan = 16;        // edges per frontier entry (64 and 8 lanes: 50,000 nodes 123 us, 16 and 16: 99)
-constexpr uint32_t kEntryLanes = 16;  // lanes per entry
 constexpr uint32_t kLongRow = 1024;  // scan: rows above are walked by the block
 constexpr uint32_t kLongList = 64;
 constexpr double kAlpha = 14.0, kBeta = 24.0;
@@ -67,31 +65,6 @@ __global__ void bfs_init_k(BfsArgs a, uint32_t source, unsigned long long edges)
   *a.st = s;
 }
 
-// Appends the lanes' new nodes (w where take) to the next frontier's list.
-__device__ __forceinline__ void bfs_append(const BfsArgs& a, int parity, bool take, uint32_t w,
-                                           uint32_t deg) {
-  const uint32_t FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  const uint32_t k = take ? (deg + kSpan - 1) / kSpan : 0u;
-  if (!__any_sync(FULL, k != 0)) return;
-  uint32_t incl = k;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(FULL, incl, o);
-    if (lane >= o) incl += t;
-  }
-  uint32_t base = 0;
-  if (lane == 31) base = atomicAdd(&a.st->entries[parity], incl);
-  base = __shfl_sync(FULL, base, 31) + incl - k;
-  if (k && k <= 32)
-    for (uint32_t i = 0; i < k; i++) a.list[parity][base + i] = make_uint2(w, i * kSpan);
-  for (uint32_t big = __ballot_sync(FULL, k > 32); big; big &= big - 1) {  // a hub: the warp's lanes together
-    const int l = __ffs(big) - 1;
-    const uint32_t bk = __shfl_sync(FULL, k, l), bb = __shfl_sync(FULL, base, l), bw = __shfl_sync(FULL, w, l);
-    for (uint32_t i = lane; i < bk; i += 32) a.list[parity][bb + i] = make_uint2(bw, i * kSpan);
-  }
-}
-
 // One step of a warp along edges: every lane has a neighbour w (or none).
 __device__ __forceinline__ void bfs_visit(const BfsArgs& a, int32_t level, bool have, uint32_t w,
                                           unsigned long long& f, unsigned long long& T) {
@@ -103,7 +76,7 @@ __device__ __forceinline__ void bfs_visit(const BfsArgs& a, int32_t level, bool 
     f++;
     T += deg;
   }
-  bfs_append(a, (level + 1) & 1, take, w, deg);
+  append_entries(a.list[(level + 1) & 1], &a.st->entries[(level + 1) & 1], take, w, deg);
 }
 
 __global__ void __launch_bounds__(kBlock) bfs_level_k(BfsArgs a) {

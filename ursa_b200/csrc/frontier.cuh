@@ -64,6 +64,38 @@ __device__ __forceinline__ uint64_t owner_in_pos(const uint64_t* __restrict__ po
   return lo;
 }
 
+// A frontier as entries (node, first slot) of at most kSpan edges each, so
+// that a hub is many entries, with kEntryLanes lanes per entry (BFS of 50,000
+// nodes with 64 edges and 8 lanes 123 us, 16 and 16: 99).
+constexpr uint32_t kSpan = 16;
+constexpr uint32_t kEntryLanes = 16;
+
+// Appends the entries of the lanes' nodes (v, of degree deg, where take) to
+// list, whose length is *count.  Called by a whole warp.
+__device__ __forceinline__ void append_entries(uint2* list, uint32_t* count, bool take, uint32_t v,
+                                               uint32_t deg) {
+  const uint32_t FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const uint32_t k = take ? (deg + kSpan - 1) / kSpan : 0u;
+  if (!__any_sync(FULL, k != 0)) return;
+  uint32_t incl = k;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(FULL, incl, o);
+    if (lane >= o) incl += t;
+  }
+  uint32_t base = 0;
+  if (lane == 31) base = atomicAdd(count, incl);
+  base = __shfl_sync(FULL, base, 31) + incl - k;
+  if (k && k <= 32)
+    for (uint32_t i = 0; i < k; i++) list[base + i] = make_uint2(v, i * kSpan);
+  for (uint32_t big = __ballot_sync(FULL, k > 32); big; big &= big - 1) {  // a hub: the warp's lanes together
+    const int l = __ffs(big) - 1;
+    const uint32_t bk = __shfl_sync(FULL, k, l), bb = __shfl_sync(FULL, base, l), bv = __shfl_sync(FULL, v, l);
+    for (uint32_t i = lane; i < bk; i += 32) list[bb + i] = make_uint2(bv, i * kSpan);
+  }
+}
+
 // Device buffers reused across the levels of one traversal.
 struct FrontierBufs {
   Scratch<uint32_t> F, N;   // current / next frontier (capacity n)
