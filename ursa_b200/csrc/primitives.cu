@@ -18,6 +18,16 @@ constexpr int kScanTile = 2048;  // 256 threads x 8 items
 constexpr int kRadixItems = 16;  // per thread
 constexpr int kRadixTile = kBlock * kRadixItems;  // 4096
 constexpr int kWarps = kBlock / 32;
+constexpr int kDownBlock = 512;  // threads of a tile's block in radix_carry_k
+constexpr int kDownItems = kRadixTile / kDownBlock;
+constexpr int kDownWarps = kDownBlock / 32;
+// From 3 * 2^24 rows (a 200 MB column: its gather leaves L2) to 2^30 (above,
+// two buffers more would count) the gathered column travels with the pairs: at
+// 65M rows three passes take 600 + 620 + 535 us against 460 + 466 + 1,187 with
+// the gather in the last one (a build and a PageRank 9.07 -> 8.07 ms).  Where
+// the rows come sorted by source the out-CSR's gather is a stream: there the
+// two are even at 67M rows, and the gather is 1% faster at 48M, 2% at 36M.
+constexpr uint64_t kCarryMin = 3ull << 24, kCarryMax = 1ull << 30;
 
 __device__ __forceinline__ int pad(int i) { return i + (i >> 5); }
 
@@ -238,6 +248,146 @@ __global__ void __launch_bounds__(kBlock) radix_downsweep_k(
   }
 }
 
+// A word from global to shared memory without a register (any 4-byte
+// alignment); waited for with tile_wait().
+__device__ __forceinline__ void tile_copy(uint32_t* dst, const uint32_t* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                   static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void tile_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// The downsweep of triples: key, value (vals_in == nullptr: the input
+// position) and a third word.  A pass is bound by shared memory (ranking and
+// staging, some 40 accesses of a warp per 32 items) and by the loads'
+// latency, not by the 24 bytes an item moves.  So the values and the third
+// words cross to shared memory while the keys are ranked, and only the keys'
+// ranks are held in registers.
+struct CarrySmem {
+  uint32_t stage[kRadixTile];
+  uint32_t vals[kRadixTile];
+  uint32_t other[kRadixTile];
+  uint32_t gofs[256];  // global start of the digit, less its start in the tile
+  uint16_t wcnt[kDownWarps][256];
+  uint32_t warp_sum[8];
+};
+
+__global__ void __launch_bounds__(kDownBlock, 3) radix_carry_k(
+    const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
+    const uint32_t* __restrict__ other_in, uint64_t n, int shift, uint32_t mask,
+    const uint32_t* __restrict__ hist_scanned, uint32_t num_tiles, uint32_t* __restrict__ keys_out,
+    uint32_t* __restrict__ vals_out, uint32_t* __restrict__ other_out) {
+  extern __shared__ __align__(16) unsigned char carry_sm[];
+  CarrySmem& sm = *reinterpret_cast<CarrySmem*>(carry_sm);
+  const uint32_t tile = blockIdx.x;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint32_t lt = (1u << lane) - 1u;
+  // Warp w owns the contiguous sub-tile [w*256, (w+1)*256); round i covers
+  // items w*256 + i*32 + lane, so (round, lane) order is input order.
+  const uint64_t tile0 = (uint64_t)tile * kRadixTile;
+  const uint32_t item0 = w * (32 * kDownItems) + lane;
+  const uint32_t tile_n = (uint32_t)(n - tile0 < (uint64_t)kRadixTile ? n - tile0 : kRadixTile);
+  uint32_t k[kDownItems], p[kDownItems];
+#pragma unroll
+  for (int i = 0; i < kDownItems; i++) {
+    const uint32_t it = item0 + i * 32;
+    k[i] = it < tile_n ? __ldg(&keys_in[tile0 + it]) : 0u;
+  }
+#pragma unroll
+  for (int i = 0; i < kDownItems; i++) {
+    const uint32_t it = item0 + i * 32;
+    if (it < tile_n) {
+      if (vals_in) tile_copy(&sm.vals[it], &vals_in[tile0 + it]);
+      tile_copy(&sm.other[it], &other_in[tile0 + it]);
+    }
+  }
+  const uint32_t digit = threadIdx.x;  // of the first 256 threads
+  const uint32_t g = digit < 256 ? hist_scanned[(uint64_t)digit * num_tiles + tile] : 0u;
+  for (int i = lane; i < 256; i += 32) sm.wcnt[w][i] = 0;
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < kDownItems; i++) {
+    const uint32_t d = (k[i] >> shift) & mask;
+    const bool valid = item0 + i * 32 < tile_n;
+    const uint32_t peers = __match_any_sync(0xffffffffu, valid ? d : 256u);
+    const uint32_t before = valid ? sm.wcnt[w][d] : 0u;
+    __syncwarp();
+    const uint32_t rank = __popc(peers & lt);
+    if (valid && rank == 0) sm.wcnt[w][d] = (uint16_t)(before + __popc(peers));
+    __syncwarp();
+    p[i] = before + rank;
+  }
+  __syncthreads();
+  // Per digit: the tile's total, and each warp's start in the ordered tile.
+  uint32_t sum = 0, incl = 0;
+  if (digit < 256) {
+#pragma unroll
+    for (int ww = 0; ww < kDownWarps; ww++) sum += sm.wcnt[ww][digit];
+    incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += x;
+    }
+    if (lane == 31) sm.warp_sum[w] = incl;
+  }
+  __syncthreads();
+  if (digit < 256) {
+    uint32_t run = incl - sum;
+    for (int ww = 0; ww < w; ww++) run += sm.warp_sum[ww];
+    sm.gofs[digit] = g - run;
+#pragma unroll
+    for (int ww = 0; ww < kDownWarps; ww++) {
+      const uint32_t x = sm.wcnt[ww][digit];
+      sm.wcnt[ww][digit] = (uint16_t)run;
+      run += x;
+    }
+  }
+  __syncthreads();
+  // the tile in digit order, so that it is written in one run per digit
+#pragma unroll
+  for (int i = 0; i < kDownItems; i++) {
+    p[i] += sm.wcnt[w][(k[i] >> shift) & mask];
+    if (item0 + i * 32 < tile_n) sm.stage[p[i]] = k[i];
+  }
+  __syncthreads();
+  uint32_t dest[kDownItems];
+#pragma unroll
+  for (int j = 0; j < kDownItems; j++) {
+    const uint32_t i = j * kDownBlock + threadIdx.x;
+    if (i < tile_n) {
+      const uint32_t key = sm.stage[i];
+      dest[j] = sm.gofs[(key >> shift) & mask] + i;
+      keys_out[dest[j]] = key;
+    }
+  }
+  tile_wait();
+  __syncthreads();  // every copy has landed, and the keys have been read
+#pragma unroll
+  for (int i = 0; i < kDownItems; i++) {
+    const uint32_t it = item0 + i * 32;
+    if (it < tile_n) sm.stage[p[i]] = vals_in ? sm.vals[it] : (uint32_t)(tile0 + it);
+  }
+  __syncthreads();  // the values have been read from sm.vals, too
+#pragma unroll
+  for (int j = 0; j < kDownItems; j++) {
+    const uint32_t i = j * kDownBlock + threadIdx.x;
+    if (i < tile_n) vals_out[dest[j]] = sm.stage[i];
+  }
+#pragma unroll
+  for (int i = 0; i < kDownItems; i++) {
+    const uint32_t it = item0 + i * 32;
+    if (it < tile_n) sm.vals[p[i]] = sm.other[it];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < kDownItems; j++) {
+    const uint32_t i = j * kDownBlock + threadIdx.x;
+    if (i < tile_n) other_out[dest[j]] = sm.vals[i];
+  }
+}
+
 __global__ void offsets_k(const uint32_t* __restrict__ keys, uint64_t m, uint64_t n,
                           uint32_t* __restrict__ off) {
   for (uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; u <= n;
@@ -252,6 +402,21 @@ __global__ void offsets_k(const uint32_t* __restrict__ keys, uint64_t m, uint64_
     }
     off[u] = (uint32_t)lo;
   }
+}
+
+// radix_carry_k's shared memory is above the default limit: raised once per
+// device.
+void carry_allow_smem() {
+  static std::mutex mu;
+  static bool done[64] = {false};
+  int dev = 0;
+  UG_CUDA(cudaGetDevice(&dev));
+  UG_CHECK(dev >= 0 && dev < 64, URSA_GPU_EINVAL, "device index out of range");
+  std::lock_guard<std::mutex> g(mu);
+  if (done[dev]) return;
+  UG_CUDA(cudaFuncSetAttribute(radix_carry_k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)sizeof(CarrySmem)));
+  done[dev] = true;
 }
 
 }  // namespace
@@ -274,17 +439,18 @@ void radix_sort_pairs(const uint32_t* keys_in, const uint32_t* vals_in, uint64_t
   int passes = key_bits <= 8 ? 1 : (key_bits + 7) / 8;
   uint32_t num_tiles = (uint32_t)((n + kRadixTile - 1) / kRadixTile);
   Scratch<uint32_t> hist((size_t)256 * num_tiles, s);
-  Scratch<uint32_t> kb[2], vb[2];
-  if (passes > 1) {
-    kb[0].alloc(n, s);
-    vb[0].alloc(n, s);
-    if (passes > 2) {
-      kb[1].alloc(n, s);
-      vb[1].alloc(n, s);
-    }
+  // a column that still arrives is gathered in the last pass
+  const bool carry = gather_src && !gather_ready && n >= kCarryMin && n <= kCarryMax;
+  if (carry) carry_allow_smem();
+  Scratch<uint32_t> kb[2], vb[2], ob[2];
+  for (int i = 0; i < 2 && i < passes - 1; i++) {
+    kb[i].alloc(n, s);
+    vb[i].alloc(n, s);
+    if (carry) ob[i].alloc(n, s);
   }
   const uint32_t* kin = keys_in;
   const uint32_t* vin = vals_in;
+  const uint32_t* oin = gather_src;
   for (int p = 0; p < passes; p++) {
     int shift = 8 * p;
     int bits = key_bits - shift;
@@ -299,9 +465,16 @@ void radix_sort_pairs(const uint32_t* keys_in, const uint32_t* vals_in, uint64_t
     UG_LAUNCH_CHECK();
     exclusive_scan_u32(hist.get(), hist.get(), (uint64_t)256 * num_tiles, nullptr, s);
     if (last && gather_ready) UG_CUDA(cudaStreamWaitEvent(s, gather_ready, 0));
-    radix_downsweep_k<<<num_tiles, kBlock, 0, s>>>(kin, vin, n, shift, mask, hist.get(), num_tiles,
-                                                   kout, vout, last ? gather_src : nullptr,
-                                                   gather_out);
+    if (carry) {
+      uint32_t* oout = last ? gather_out : ob[p & 1].get();
+      radix_carry_k<<<num_tiles, kDownBlock, sizeof(CarrySmem), s>>>(
+          kin, vin, oin, n, shift, mask, hist.get(), num_tiles, kout, vout, oout);
+      oin = oout;
+    } else {
+      radix_downsweep_k<<<num_tiles, kBlock, 0, s>>>(kin, vin, n, shift, mask, hist.get(), num_tiles,
+                                                     kout, vout, last ? gather_src : nullptr,
+                                                     gather_out);
+    }
     UG_LAUNCH_CHECK();
     kin = kout;
     vin = vout;
