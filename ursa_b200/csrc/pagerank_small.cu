@@ -109,6 +109,7 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1) pr_
   __shared__ uint32_t s_rows[kCtas + 1];
   __shared__ uint32_t s_warp[kWarps];
   cg::cluster_group cluster = cg::this_cluster();
+  cluster.barrier_arrive();  // waited for before the first write to another CTA's shared memory
   const uint32_t me = cluster.block_rank();
   const int lane = threadIdx.x & 31;
   if (threadIdx.x <= kCtas) s_rows[threadIdx.x] = threadIdx.x == kCtas ? a.n : first_row(a, threadIdx.x);
@@ -141,6 +142,10 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1) pr_
     const uint32_t d = a.out_off[u + 1] - a.out_off[u];
     x0[u] = d ? (float)(first / (double)d) : 0.f;
   }
+  // A CTA's shared memory may be written from another only once it has
+  // started; the arrival was at the kernel's entry, so the loads above hide
+  // the wait.
+  cluster.barrier_wait();
   publish(cluster, part[0], acc);
   __syncthreads();
   // rows by length, in row order within a length: a lane's rows, and so the
