@@ -13,9 +13,10 @@
 // The arithmetic is pagerank.cu's, operation for operation: f32 shares, a row
 // of up to 64 in-edges summed by one lane in CSR order with a compensated f32
 // pair, longer rows in pieces of 128 edges combined in that kernel's order;
-// f64 ranks, residual and dangling mass.  So both kernels give the same ranks
-// bit for bit on the graphs compared.  A call on 1,000 nodes, 10,000 edges:
-// 234 us before, 69 now; R-MAT with 14,336 nodes and 140,000 edges: 287 and
+// f64 ranks; residual and dangling mass summed exactly, in fixed point.  So
+// both kernels give the same ranks bit for bit on the graphs compared.  A call
+// on 1,000 nodes, 10,000 edges: 234 us before, 73 now (70 with f64 sums, which
+// depend on their order); R-MAT with 14,336 nodes and 140,000 edges: 287 and
 // 200.  What is left is the launch and, per iteration, the chain of one row's
 // additions, two block-wide waits and the cluster barrier (about 4 us).
 #include <cooperative_groups.h>
@@ -23,6 +24,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "fixedpoint.cuh"
 #include "topo.cuh"
 
 namespace cg = cooperative_groups;
@@ -41,7 +43,8 @@ constexpr int kWarps = kThreads / 32;
 constexpr uint64_t kMaxNodes = 14336;
 constexpr uint64_t kMaxEdges = 1u << 18;  // R-MAT with 14,336 nodes: 224,000 edges 236 us (275), twice that slower
 constexpr uint64_t kMaxPieces = (2 * kMaxEdges + kMaxNodes) / 8 / 64 + kMaxEdges / 128 + 2;
-constexpr size_t kSmemBytes = 227u * 1024u - 9u * 1024u;  // 8 KB and more are static
+constexpr size_t kSmemBytes = 227u * 1024u - 3u * 1024u;  // under 2 KB are static
+static_assert(kWarps == 32, "one warp sums the warps' sums");
 static_assert(8 * kMaxNodes + 18 * (kMaxNodes / 4 + 2) + 12 * kMaxPieces + 32 <= kSmemBytes, "a CTA's rows fit");
 constexpr uint32_t kShort = 8;     // rows up to this are kept together, so that lanes end together
 constexpr uint32_t kDirect = 64;   // rows up to this: one lane
@@ -73,39 +76,54 @@ __device__ uint32_t first_row(const SmallArgs& a, uint32_t c) {
   return lo;
 }
 
-// Sums over the warp, fixed order; valid in every lane.
-__device__ __forceinline__ double2 warp_sum(double2 v) {
+// (residual, dangling mass) in fixed point, as in pagerank.cu: exact, in any
+// order.
+struct Sums {
+  u128 delta, dang;
+};
+
+// Sums over the warp, valid in every lane: limbs of 26 bits, whose 32-lane
+// sums fit the 32 bits of a warp-wide add (shuffles of whole words: 90 us
+// against 73 for a call on 1,000 nodes).
+__device__ __forceinline__ u128 warp_sum(u128 v) {
+  constexpr int kBits = 26;
+  if (!__any_sync(0xffffffffu, v != 0)) return 0;  // warps without rows, graphs without dangling nodes
+  u128 t = 0;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+  for (int i = 0; i * kBits < 128; i++) {
+    const uint32_t limb = (uint32_t)(v >> (i * kBits)) & ((1u << kBits) - 1u);
+    t += (u128)__reduce_add_sync(0xffffffffu, limb) << (i * kBits);
   }
-  return v;
+  return t;
 }
 
-// Every warp's sums, put into every CTA's table (lane c writes CTA c's).
-__device__ __forceinline__ void publish(cg::cluster_group& cluster, double2* table, double2 v) {
-  v = warp_sum(v);
+__device__ __forceinline__ Sums warp_sum(Sums v) { return Sums{warp_sum(v.delta), warp_sum(v.dang)}; }
+
+// The CTA's sums, put into every CTA's table (lane c of warp 0 writes CTA c's).
+__device__ __forceinline__ void publish(cg::cluster_group& cluster, FxPair* table, FxPair* warps, Sums v) {
   const uint32_t lane = threadIdx.x & 31;
-  if (lane < kCtas)
-    cluster.map_shared_rank(table, lane)[cluster.block_rank() * kWarps + (threadIdx.x >> 5)] = v;
+  v = warp_sum(v);
+  if (lane == 0) warps[threadIdx.x >> 5] = fx_pack(v.delta, v.dang);
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  const FxPair w = warps[lane];
+  v = warp_sum(Sums{fx_delta(w), fx_dang(w)});
+  if (lane < kCtas) cluster.map_shared_rank(table, lane)[cluster.block_rank()] = fx_pack(v.delta, v.dang);
 }
 
 // The table's total, the same in every thread of the cluster.
-__device__ __forceinline__ double2 total(const double2* table) {
-  double2 t = make_double2(0.0, 0.0);
-#pragma unroll
-  for (int c = 0; c < kCtas; c++) {
-    const double2 v = table[c * kWarps + (threadIdx.x & 31)];
-    t.x += v.x;
-    t.y += v.y;
-  }
-  return warp_sum(t);
+__device__ __forceinline__ double2 total(const FxPair* table) {
+  const uint32_t lane = threadIdx.x & 31;
+  Sums t{0, 0};
+  if (lane < kCtas) t = Sums{fx_delta(table[lane]), fx_dang(table[lane])};
+  t = warp_sum(t);
+  return make_double2(fx_value(t.delta), fx_value(t.dang));
 }
 
 __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1) pr_small_k(SmallArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ double2 part[2][kCtas * kWarps];  // (residual, dangling mass) of every warp, by parity
+  __shared__ FxPair part[2][kCtas];  // every CTA's sums, by parity
+  __shared__ FxPair warps[kWarps];   // this CTA's, per warp
   __shared__ uint32_t s_rows[kCtas + 1];
   __shared__ uint32_t s_warp[kWarps];
   cg::cluster_group cluster = cg::this_cluster();
@@ -128,7 +146,7 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1) pr_
   const double nf = (double)a.n;
   const double first = 1.0 / nf;
   if (threadIdx.x == 0) off[rows] = edges;
-  double2 acc = make_double2(0.0, 0.0);  // residual, dangling mass
+  Sums acc{0, 0};
   for (uint32_t r = threadIdx.x; r < rows; r += kThreads) {
     const uint32_t u = r0 + r;
     const uint32_t b = a.in_off[u];
@@ -136,7 +154,7 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1) pr_
     const uint32_t d = a.out_off[u + 1] - a.out_off[u];
     div[r] = d;
     rank[r] = first;
-    if (d == 0) acc.y += first;
+    if (d == 0) acc.dang += fx_of(first);
   }
   for (uint32_t u = threadIdx.x; u < a.n; u += kThreads) {  // every CTA fills its own copy
     const uint32_t d = a.out_off[u + 1] - a.out_off[u];
@@ -146,7 +164,7 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1) pr_
   // started; the arrival was at the kernel's entry, so the loads above hide
   // the wait.
   cluster.barrier_wait();
-  publish(cluster, part[0], acc);
+  publish(cluster, part[0], warps, acc);
   __syncthreads();
   // rows by length, in row order within a length: a lane's rows, and so the
   // order of the sums below, are the same in every run
@@ -222,13 +240,13 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1) pr_
     const double dm = sums.y;
     // base = (1-d)/n + d*dangling_mass/n   (pagerank.rs:79)
     const double base = __dadd_rn(__ddiv_rn(1.0 - a.damping, nf), __ddiv_rn(__dmul_rn(a.damping, dm), nf));
-    acc = make_double2(0.0, 0.0);
+    acc = Sums{0, 0};
     auto finish = [&](uint32_t r, double sum) {  // next[u] = base + d * contrib(u)  (:81-83)
       const double nx = __dadd_rn(base, __dmul_rn(a.damping, sum));
-      acc.x += fabs(nx - rank[r]);
+      acc.delta += fx_of(fabs(__dsub_rn(nx, rank[r])));
       rank[r] = nx;
       const uint32_t d = div[r];
-      if (d == 0) acc.y += nx;
+      if (d == 0) acc.dang += fx_of(nx);
       const float share = d ? (float)(nx / (double)d) : 0.f;
 #pragma unroll
       for (int c = 0; c < kCtas; c++) cluster.map_shared_rank(nxt, c)[r0 + r] = share;
@@ -284,7 +302,7 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1) pr_
         if (lane == 0) finish(longs[i], f2_value(v));
       }
     }
-    publish(cluster, part[(it + 1) & 1], acc);
+    publish(cluster, part[(it + 1) & 1], warps, acc);
     cluster.sync();  // new shares and partial sums are in place everywhere
     sums = total(part[(it + 1) & 1]);
     delta = sums.x;
