@@ -16,6 +16,7 @@
 // hash slot, flushed once per v).  Integer results are order-independent, so
 // the counts are bit-identical to the reference.
 #include "frontier.cuh"
+#include "tclist.h"
 #include "tcstream.cuh"
 
 namespace ug {
@@ -54,13 +55,12 @@ __device__ __forceinline__ uint32_t tc_hash(uint32_t w, uint32_t bits) {
   return (w * 0x9E3779B1u) >> (32 - bits);
 }
 
-// N+(v) of up to kTcSearchMax elements is searched where it lies, a lane per
-// probe whatever its v; up to kTcWarpMax a warp's hash table; larger ones a
-// block's.  Most vertices have short lists and few probes: a table for each
+// N+(v) of up to search_max elements (tclist.h: 24 below 2^30 edges) is
+// searched where it lies, a lane per probe whatever its v; up to kTcWarpMax a
+// warp's hash table; larger ones a block's.  Most vertices have short lists and few probes: a table for each
 // of them was all latency (1,024 probes could take 300 tables).  Searched up
 // to 16 / 24 / 32 elements: R-MAT-16 884 / 892 / 935 us a call, a Poisson graph
 // of mean degree 32 3,345 / 3,168 / 3,129.
-constexpr uint32_t kTcSearchMax = 24;  // five halvings
 constexpr uint32_t kTcWarpMax = 256;
 constexpr uint32_t kTcBlockWarps = 8;
 constexpr uint32_t kTcMidSlots = 2048;  // a block's table in shared memory
@@ -70,15 +70,13 @@ constexpr uint32_t kTcMidSlots = 2048;  // a block's table in shared memory
 // size (an entry's probes stay together) whatever vertices they span: a
 // vertex's in-list is cut where it is long, and the next table starts where
 // the last one ended.  At most kTcChunks chunks, so that the last ones end
-// together on a large graph; at least kTcMinWork units of kTcUnit probes
-// each.  (Pieces of up to 16K probes of one in-list, sixteen to a grab, left
+// together on a large graph; at least kTcMinWork probes each.  (Pieces of up to 16K probes of one in-list, sixteen to a grab, left
 // R-MAT-16's 7,000 warps waiting for the few that drew the hubs: 4.85 ms of
 // warp tables against 0.41; one cut over all vertices left them skipping
 // thousands of other kinds' lists: 13.7 ms of block tables on R-MAT-20 against
 // 3.6.)
 constexpr uint32_t kTcChunks[2] = {1u << 17, 1u << 13};
-constexpr uint64_t kTcUnit = 256;
-constexpr uint64_t kTcMinWork[2] = {4, 32};
+constexpr uint64_t kTcMinWork[2] = {1024, 8192};
 constexpr uint32_t kTcSearchEntries = 256;  // most in-list entries per grab of a searching warp
 constexpr int kTcKinds = 2;                 // warp tables, block tables
 
@@ -183,10 +181,8 @@ struct TcList {
   uint32_t* chunk_i;
   uint32_t* chunk_e;
 };
-// Device words of a call: per kind, vertices << 38 | work units of the list
-// (so at most 2^26 vertices with more than 32 of below 2^31 edges, and 2^46
-// probes), chunks in use, and the grab counters.
-constexpr int kTcWorkBits = 38;
+// Device words of a call: per kind, the list's vertices and work (tclist.h),
+// chunks in use, and the grab counters.
 struct TcCtl {
   unsigned long long size[kTcKinds];
   unsigned long long next[kTcKinds + 1];
@@ -202,6 +198,7 @@ struct TcArgs {
   const uint32_t* in_rank;    // ... and the rank of the list
   const uint32_t* vertex_of;  // rank -> original id
   uint64_t entries;           // in-list entries of all ranks
+  uint32_t search_max;
   uint32_t grab;              // ... taken at a time by a searching warp
   TcList list;                // this launch's kind
   int kind;
@@ -233,7 +230,7 @@ __device__ __forceinline__ uint32_t tc_bits(uint32_t dv) {
   return max(3u, 32u - (uint32_t)__clz(2 * dv - 1));
 }
 
-// Middle vertices with |N+(v)| <= kTcSearchMax: a warp takes 32 entries at a
+// Middle vertices with |N+(v)| <= search_max: a warp takes 32 entries at a
 // time whatever their v; each probe is searched in N+(v) by bisection.
 __global__ void __launch_bounds__(256) tc_middle_search_k(TcArgs a) {
   __shared__ uint32_t pack[8][32];
@@ -251,7 +248,7 @@ __global__ void __launch_bounds__(256) tc_middle_search_k(TcArgs a) {
         v = a.vertex_of[a.in_rank[e + lane]];
         ob = a.off[v];
         dv = a.off[v + 1] - ob;
-        if (dv != 0 && dv <= kTcSearchMax) {
+        if (dv != 0 && dv <= a.search_max) {
           u = a.in_src[e + lane];
           b = a.in_pos[e + lane] + 1;
           len = a.off[u + 1] - b;
@@ -544,7 +541,7 @@ __global__ void entry_work_k(const uint32_t* __restrict__ off, const uint32_t* _
 // the vertices' places and the work before them together.
 __global__ void tc_lists_k(const uint32_t* __restrict__ in_off, const uint32_t* __restrict__ off,
                            const uint32_t* __restrict__ vertex_of, const uint64_t* __restrict__ wp,
-                           uint64_t n, TcList warp_list, TcList block_list, TcCtl* ctl) {
+                           uint64_t n, TcSplit split, TcList warp_list, TcList block_list, TcCtl* ctl) {
   const uint32_t FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -557,9 +554,9 @@ __global__ void tc_lists_k(const uint32_t* __restrict__ in_off, const uint32_t* 
       if (b != e) {
         const uint32_t v = vertex_of[r];
         const uint32_t dv = off[v + 1] - off[v];
-        if (dv > kTcSearchMax) {
+        if (dv > split.search_max) {
           kind = dv > kTcWarpMax ? 1 : 0;
-          x = (1ull << kTcWorkBits) + (wp[e] - wp[b]) / kTcUnit + 1;
+          x = (1ull << kTcWorkBits) + ((wp[e] - wp[b]) >> split.unit_shift) + 1;
         }
       }
     }
@@ -591,7 +588,7 @@ __global__ void tc_lists_k(const uint32_t* __restrict__ in_off, const uint32_t* 
 // or after.
 __global__ void tc_chunks_k(const uint32_t* __restrict__ in_off, const uint64_t* __restrict__ wp,
                             TcList list, int kind, uint64_t min_work,
-                            uint64_t max_chunks, TcCtl* ctl) {
+                            uint64_t max_chunks, uint32_t unit_shift, TcCtl* ctl) {
   const unsigned long long size = ctl->size[kind];
   const uint32_t count = (uint32_t)(size >> kTcWorkBits);
   const uint64_t work = size & ((1ull << kTcWorkBits) - 1);
@@ -612,7 +609,7 @@ __global__ void tc_chunks_k(const uint32_t* __restrict__ in_off, const uint64_t*
     }
     const uint32_t r = list.rank[lo];
     uint32_t e = in_off[r], end = in_off[r + 1];
-    const uint64_t cut = wp[e] + (want - list.at[lo]) * kTcUnit;
+    const uint64_t cut = wp[e] + ((want - list.at[lo]) << unit_shift);
     while (e < end) {
       const uint32_t mid = e + ((end - e) >> 1);
       if (wp[mid] < cut) e = mid + 1; else end = mid;
@@ -769,7 +766,9 @@ void triangle_count_run(TopoImpl* t, uint32_t* d_tri, cudaStream_t s) {
   UG_LAUNCH_CHECK();
   UG_CUDA(cudaMemsetAsync(wp.get() + mo, 0, sizeof(uint64_t), s));
   exclusive_scan_u64(wp.get(), wp.get(), mo + 1, nullptr, s);
-  const uint64_t listed = std::min<uint64_t>(n, mo / kTcSearchMax + 1);  // at most, of a kind
+  UG_CHECK(mo <= kTcMaxEdges, URSA_GPU_EINVAL, "triangle count: too many undirected edges");
+  const TcSplit split = tc_split(mo);
+  const uint64_t listed = std::min<uint64_t>(n, tc_max_listed(mo) + 1);  // at most, of a kind
   Scratch<uint32_t> ranks(kTcKinds * listed, s), chunk_at(2 * (kTcChunks[0] + kTcChunks[1] + 2ull), s);
   Scratch<uint64_t> before(kTcKinds * listed, s);
   Scratch<TcCtl> ctl(1, s);
@@ -780,11 +779,12 @@ void triangle_count_run(TopoImpl* t, uint32_t* d_tri, cudaStream_t s) {
     lists[k] = TcList{ranks.get() + k * listed, before.get() + k * listed, at, at + kTcChunks[k] + 1};
   }
   tc_lists_k<<<grid_for(n), kBlock, 0, s>>>(in_off.get(), o_off.get(), vertex_of.get(), wp.get(), n,
-                                            lists[0], lists[1], ctl.get());
+                                            split, lists[0], lists[1], ctl.get());
   UG_LAUNCH_CHECK();
   for (int k = 0; k < kTcKinds; k++) {
-    tc_chunks_k<<<grid_for(kTcChunks[k] + 1), kBlock, 0, s>>>(in_off.get(), wp.get(), lists[k], k,
-                                                              kTcMinWork[k], kTcChunks[k], ctl.get());
+    tc_chunks_k<<<grid_for(kTcChunks[k] + 1), kBlock, 0, s>>>(
+        in_off.get(), wp.get(), lists[k], k, kTcMinWork[k] >> split.unit_shift, kTcChunks[k],
+        split.unit_shift, ctl.get());
     UG_LAUNCH_CHECK();
   }
   uint32_t max_dv = 0;
@@ -804,11 +804,12 @@ void triangle_count_run(TopoImpl* t, uint32_t* d_tri, cudaStream_t s) {
   a.in_rank = in_rank.get();
   a.vertex_of = vertex_of.get();
   a.entries = mo;
+  a.search_max = split.search_max;
   a.list = lists[0];
   a.kind = 0;
   a.ctl = ctl.get();
   a.tri = d_tri;
-  {  // |N+(v)| <= 32: searched
+  {  // |N+(v)| <= search_max: searched
     static std::mutex mu;
     static int cache[64] = {0};
     const int per_sm = tc_blocks_per_sm(tc_middle_search_k, 256, 0, dev, cache, mu);
@@ -819,7 +820,7 @@ void triangle_count_run(TopoImpl* t, uint32_t* d_tri, cudaStream_t s) {
     count_launch();
   }
   constexpr int kSmallSlots = 2 * kTcWarpMax, kWarpsW = 8, kWarpsB = kTcBlockWarps;
-  if (max_dv > kTcSearchMax) {  // up to 256: a warp per chunk
+  if (max_dv > split.search_max) {  // up to 256: a warp per chunk
     static std::mutex mu;
     static int cache[64] = {0};
     const size_t smem = ((size_t)kWarpsW * 2 * kSmallSlots + kWarpsW * 32) * sizeof(uint32_t);
