@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(256) tc_middle_search_k(TcArgs a) {
 // warp in shared memory (kWarps warps per block).
 template <int kSlots, int kWarps>
 __global__ void __launch_bounds__(kWarps * 32) tc_middle_warp_k(TcArgs a) {
-  extern __shared__ uint32_t tc_sm[];
+  extern __shared__ __align__(16) uint32_t tc_sm[];  // read as uint4
   const uint32_t FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   uint32_t* T = tc_sm + (size_t)wid * 2 * kSlots;
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(kWarps * 32) tc_middle_warp_k(TcArgs a) {
 template <int kWarps>
 __global__ void __launch_bounds__(kWarps * 32) tc_middle_block_k(TcArgs a, uint32_t* table,
                                                                  uint32_t slots) {
-  extern __shared__ uint32_t tc_sm[];
+  extern __shared__ __align__(16) uint32_t tc_sm[];  // read as uint4
   __shared__ uint32_t pack[kWarps][32];
   __shared__ unsigned long long s_g;
   const uint32_t FULL = 0xffffffffu;
@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(kSmThreads) count_small_k(const uint32_t* __re
                                                           const uint32_t* __restrict__ o_tgt,
                                                           uint64_t n, uint32_t* __restrict__ tri,
                                                           unsigned long long* __restrict__ next) {
-  extern __shared__ uint32_t tc_sm[];
+  extern __shared__ __align__(16) uint32_t tc_sm[];
   const uint32_t FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   uint32_t* T = tc_sm + (size_t)w * kSmSlots;
