@@ -5,6 +5,7 @@
 #include <cstdlib>
 #include <initializer_list>
 
+#include "msshape.h"
 #include "tclist.h"
 
 #define EXPECT(x)                                    \
@@ -32,7 +33,26 @@ static void triangle_lists() {
   EXPECT(25 <= tc_split(ring * 25).search_max || ring < (1ull << (64 - kTcWorkBits)));
 }
 
+// Every grid fits the blocks that are resident at once, whatever the GPU (or
+// the part of one) has: the groups' blocks wait for one another.
+static void many_source_grids() {
+  using namespace ug;
+  for (uint64_t sms = 1; sms <= 160; sms++)
+    for (uint64_t per_sm : {1, 2, 4, 5, 8})
+      for (int W : {1, 4})
+        for (uint64_t n : std::initializer_list<uint64_t>{1, 31, 256, 257, 8192, 65536, 1u << 20, 1u << 21, 1u << 28})
+          for (uint64_t sources : std::initializer_list<uint64_t>{1, 64, 65, 256, 1000, 65536, 1u << 20}) {
+            const uint64_t resident = sms * per_sm;
+            const MsShape x = ms_shape(n, sources, W, resident);
+            EXPECT(x.groups >= 1 && x.group_blocks >= 1);
+            EXPECT((uint64_t)x.groups * x.group_blocks <= resident);
+            EXPECT(x.groups <= (sources + 64 * W - 1) / (64 * W) && x.groups <= kMsGroups);
+            EXPECT(x.groups == 1 || x.groups * n * W * 32 <= kMsMaskBytes);
+          }
+}
+
 int main() {
+  many_source_grids();
   triangle_lists();
   std::printf("ok\n");
 }

@@ -35,6 +35,7 @@
 #include <vector>
 
 #include "frontier.cuh"
+#include "msshape.h"
 #include "primitives.cuh"
 
 namespace ug {
@@ -46,15 +47,6 @@ constexpr int kMsWarps = kMsBlock / 32;
 constexpr int kMsOcc = 4;   // blocks per SM of the 256-source kernel (64 registers; 5 would spill)
 constexpr int kMsOcc1 = 5;  // ... of the 64-source kernel (48)
 constexpr uint64_t kMsSourcesPerLaunch = 1024;  // per group
-// A level of a small graph is too little work for the grid: on R-MAT-16 78%
-// of the warps' time was the wait at the level's barrier.  So the grid is cut
-// into groups of blocks, each with its own barrier and masks and every
-// groups-th batch: while one group waits, another one's blocks work.  R-MAT-16
-// from every node with 1 / 6 / 16 / 32 / 64 groups: 89.6 / 46.0 / 34.4 / 27.3 /
-// 20.7 ms; beyond that the masks (4 x 32 bytes a node and group) leave L2.
-constexpr uint64_t kMsGroups = 128;       // at most
-constexpr uint64_t kMsNodesPerBlock = 8192;  // at most, of a group's pass
-constexpr uint64_t kMsMaskBytes = 512ull << 20;  // of all groups
 constexpr uint64_t kMsWaitNs = 5000000000ull;  // one grid-barrier wait
 constexpr uint64_t kMsPushDiv = 8;  // push while the frontier's out-edges are below m / 8
 constexpr uint32_t kMsHub = 64;    // in-degree above which a node's scan is split
@@ -481,24 +473,17 @@ __global__ void __launch_bounds__(kMsBlock, W == 4 ? kMsOcc : kMsOcc1) ms_persis
   }
 }
 
-// Groups and blocks per group for n nodes and a number of batches.
+static_assert(kMsBlockNodes == 32 * kMsWarps, "a warp per 32 nodes");
+
+// Blocks of either variant (with and without groups) that are resident at once.
 template <int W>
-void ms_shape(uint64_t n, uint64_t n_sources, int device, MsArgs& a) {
-  int per_sm = 0;
-  UG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ms_persist_k<W, true>, kMsBlock, 0));
+uint64_t ms_resident(int device) {
+  int a = 0, b = 0;
+  UG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, ms_persist_k<W, true>, kMsBlock, 0));
+  UG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, ms_persist_k<W, false>, kMsBlock, 0));
+  const int per_sm = std::min(a, b);
   UG_CHECK(per_sm > 0, URSA_GPU_ECUDA, "msbfs: kernel cannot be resident");
-  const uint64_t cap = (uint64_t)per_sm * sm_count(device);
-  const uint64_t batches = (n_sources + 64 * W - 1) / (64 * W);
-  uint64_t groups = std::min(batches, cap * kMsNodesPerBlock / n);
-  groups = std::min({groups, kMsMaskBytes / (n * W * 32), kMsGroups});
-  groups = std::max<uint64_t>(1, groups);
-  const uint64_t rounds = (batches + groups - 1) / groups;  // as many groups as the rounds need
-  groups = (batches + rounds - 1) / rounds;
-  // one warp per 32 nodes is all a level pass uses; fewer blocks make
-  // cheaper barriers
-  const uint64_t want = (n + 32 * kMsWarps - 1) / (32 * kMsWarps);
-  a.groups = (uint32_t)groups;
-  a.group_blocks = (uint32_t)std::max<uint64_t>(1, std::min(want, cap / groups));
+  return (uint64_t)per_sm * sm_count(device);
 }
 
 template <int W>
@@ -776,10 +761,9 @@ static void msbfs_enqueue(TopoImpl* t, int dir, const uint32_t* d_src, uint64_t 
   const TopoImpl::MsHubs& hb = ensure_ms_hubs(t, dir, c, s);
   const int W = n_sources >= 256 && n <= (1ull << 21) ? 4 : 1;
   MsArgs a;
-  if (W == 4)
-    ms_shape<4>(n, n_sources, t->device, a);
-  else
-    ms_shape<1>(n, n_sources, t->device, a);
+  const MsShape shape = ms_shape(n, n_sources, W, W == 4 ? ms_resident<4>(t->device) : ms_resident<1>(t->device));
+  a.groups = shape.groups;
+  a.group_blocks = shape.group_blocks;
   const uint64_t words = a.groups * n * W;
   Scratch<unsigned long long> visited(words, s), fa(words, s), fb(words, s), acc(words, s);
   Scratch<unsigned long long> count(a.groups * 3 * (64 * W + 8), s);
