@@ -241,28 +241,17 @@ void bfs_distances_run(TopoImpl* t, uint32_t source, int dir, int32_t* d_dist, i
   bfs_init_k<<<1, kBlock, 0, s>>>(a, source, edges);
   UG_LAUNCH_CHECK();
   const unsigned grid = grid_for(n, kBlock, (unsigned)sm_count(t->device) * kBfsBlocks);
-  // the first run of levels is enough for most graphs: the answer is copied
-  // behind it, and again if it was not
-  int run = 8;
-  bool copied = false;
-  while (true) {
+  uint32_t mode = kList;
+  for (int run = 8; mode != kDone; run = run < 64 ? 2 * run : run) {
     for (int i = 0; i < run; i++) {
       bfs_level_k<<<grid, kBlock, 0, s>>>(a);
       UG_LAUNCH_CHECK();
     }
-    const bool speculate = run == 8;
-    uint32_t mode = 0;
+    // a copy to pageable memory returns once it is done: the levels are over
     UG_CUDA(cudaMemcpyAsync(&mode, &st.get()->mode, sizeof(mode), cudaMemcpyDeviceToHost, s));
-    if (speculate) copy();
-    UG_CUDA(cudaStreamSynchronize(s));
-    copied = speculate;
-    if (mode == kDone) break;
-    run = run < 64 ? 2 * run : run;
   }
-  if (!copied) {
-    copy();
-    UG_CUDA(cudaStreamSynchronize(s));
-  }
+  copy();
+  UG_CUDA(cudaStreamSynchronize(s));
 }
 
 }  // namespace ug
