@@ -19,6 +19,8 @@
 //     at a time; only counts are kept;
 //   scan: the first top-down level after pulling: nodes on the last level are
 //     found by scanning dist, 32 at a time, and expanded as they are found.
+#include <algorithm>
+
 #include "frontier.cuh"
 
 namespace ug {
@@ -29,6 +31,9 @@ constexpr uint32_t kLongRow = 1024;  // scan: rows above are walked by the block
 constexpr uint32_t kLongList = 64;
 constexpr double kAlpha = 14.0, kBeta = 24.0;
 constexpr int kBfsBlocks = 8;  // per SM
+// The grid has a thread per node, or per this many edges: a level's list can
+// hold them all (256 nodes, 50M edges: 951 us with one block, 123 so).
+constexpr uint64_t kBfsLaneEdges = 64;
 
 enum Mode : uint32_t { kList = 0, kPull = 1, kScan = 2, kDone = 3 };
 
@@ -37,7 +42,7 @@ struct BfsState {
   int32_t level;  // of the frontier
   uint32_t entries[2];  // frontier entries, by level parity
   unsigned ticket;
-  uint32_t pad;
+  uint32_t limit;  // entries from which the next level is a pull
   unsigned long long f, left;          // the frontier's nodes; edges not yet walked from
   unsigned long long next_f, next_T;   // being counted: the next frontier's nodes and edges
 };
@@ -49,6 +54,14 @@ struct BfsArgs {
   uint2* list[2];  // by level parity
   BfsState* st;
 };
+
+// With this many entries the next frontier's edges pass left / kAlpha (at most
+// one entry a node is not full), so it is pulled and nobody reads its list.
+// (256 nodes, 50M edges, both directions: 257 us with all of them written, a
+// warp a hub, 150 so.)
+__device__ __forceinline__ uint32_t bfs_limit(uint64_t n, unsigned long long left) {
+  return (uint32_t)min(0xFFFFFFFFull, n + left / (unsigned long long)(kAlpha * kSpan) + 2ull);
+}
 
 __global__ void bfs_init_k(BfsArgs a, uint32_t source, unsigned long long edges) {
   const uint32_t deg = dv_deg(a.fw, source);
@@ -62,11 +75,12 @@ __global__ void bfs_init_k(BfsArgs a, uint32_t source, unsigned long long edges)
   s.entries[0] = k;
   s.f = 1;
   s.left = edges - (pull ? 0 : deg);
+  s.limit = bfs_limit(a.n, s.left);
   *a.st = s;
 }
 
 // One step of a warp along edges: every lane has a neighbour w (or none).
-__device__ __forceinline__ void bfs_visit(const BfsArgs& a, int32_t level, bool have, uint32_t w,
+__device__ __forceinline__ void bfs_visit(const BfsArgs& a, int32_t level, uint32_t limit, bool have, uint32_t w,
                                           unsigned long long& f, unsigned long long& T) {
   bool take = false;
   uint32_t deg = 0;
@@ -76,7 +90,7 @@ __device__ __forceinline__ void bfs_visit(const BfsArgs& a, int32_t level, bool 
     f++;
     T += deg;
   }
-  append_entries(a.list[(level + 1) & 1], &a.st->entries[(level + 1) & 1], take, w, deg);
+  append_entries(a.list[(level + 1) & 1], &a.st->entries[(level + 1) & 1], take, w, deg, limit);
 }
 
 __global__ void __launch_bounds__(kBlock) bfs_level_k(BfsArgs a) {
@@ -89,6 +103,7 @@ __global__ void __launch_bounds__(kBlock) bfs_level_k(BfsArgs a) {
   const uint64_t gtid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint64_t nthr = (uint64_t)gridDim.x * blockDim.x;
   unsigned long long f = 0, T = 0;  // this thread's new nodes and their edges
+  const uint32_t limit = sp->limit;
   if (mode == kList) {
     const uint32_t count = sp->entries[level & 1];
     const uint2* list = a.list[level & 1];
@@ -106,7 +121,7 @@ __global__ void __launch_bounds__(kBlock) bfs_level_k(BfsArgs a) {
       }
       while (__any_sync(FULL, j < end)) {
         const bool have = j < end;
-        bfs_visit(a, level, have, have ? dv_nbr(a.fw, u, j) : 0u, f, T);
+        bfs_visit(a, level, limit, have, have ? dv_nbr(a.fw, u, j) : 0u, f, T);
         j += kEntryLanes;
       }
     }
@@ -159,7 +174,7 @@ __global__ void __launch_bounds__(kBlock) bfs_level_k(BfsArgs a) {
         const uint32_t u = __shfl_sync(FULL, (uint32_t)v, l), d = __shfl_sync(FULL, deg, l);
         for (uint32_t j0 = 0; j0 < d; j0 += 32) {
           const bool have = j0 + lane < d;
-          bfs_visit(a, level, have, have ? dv_nbr(a.fw, u, j0 + lane) : 0u, f, T);
+          bfs_visit(a, level, limit, have, have ? dv_nbr(a.fw, u, j0 + lane) : 0u, f, T);
         }
       }
     }
@@ -169,7 +184,7 @@ __global__ void __launch_bounds__(kBlock) bfs_level_k(BfsArgs a) {
       const uint32_t u = longs[i], d = dv_deg(a.fw, u);
       for (uint32_t j0 = 0; j0 < d; j0 += blockDim.x) {
         const bool have = j0 + threadIdx.x < d;
-        bfs_visit(a, level, have, have ? dv_nbr(a.fw, u, j0 + threadIdx.x) : 0u, f, T);
+        bfs_visit(a, level, limit, have, have ? dv_nbr(a.fw, u, j0 + threadIdx.x) : 0u, f, T);
       }
     }
   }
@@ -205,6 +220,7 @@ __global__ void __launch_bounds__(kBlock) bfs_level_k(BfsArgs a) {
   if (!pull && (double)nT > (double)left / kAlpha) pull = true;
   s->mode = nf == 0 || nT == 0 ? kDone : pull ? kPull : mode == kPull ? kScan : kList;
   s->left = pull ? left : left - min(left, nT);
+  s->limit = bfs_limit(a.n, s->left);
   s->f = nf;
   s->level = level + 1;
   s->entries[level & 1] = 0;  // the list after the next
@@ -240,7 +256,8 @@ void bfs_distances_run(TopoImpl* t, uint32_t source, int dir, int32_t* d_dist, i
   a.st = st.get();
   bfs_init_k<<<1, kBlock, 0, s>>>(a, source, edges);
   UG_LAUNCH_CHECK();
-  const unsigned grid = grid_for(n, kBlock, (unsigned)sm_count(t->device) * kBfsBlocks);
+  const unsigned grid = grid_for(std::max(n, edges / kBfsLaneEdges), kBlock,
+                                 (unsigned)sm_count(t->device) * kBfsBlocks);
   uint32_t mode = kList;
   for (int run = 8; mode != kDone; run = run < 64 ? 2 * run : run) {
     for (int i = 0; i < run; i++) {

@@ -71,9 +71,10 @@ constexpr uint32_t kSpan = 16;
 constexpr uint32_t kEntryLanes = 16;
 
 // Appends the entries of the lanes' nodes (v, of degree deg, where take) to
-// list, whose length is *count.  Called by a whole warp.
+// list, whose length is *count; those that would bring it to `limit` or more
+// are counted and not written.  Called by a whole warp.
 __device__ __forceinline__ void append_entries(uint2* list, uint32_t* count, bool take, uint32_t v,
-                                               uint32_t deg) {
+                                               uint32_t deg, uint32_t limit = 0xFFFFFFFFu) {
   const uint32_t FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const uint32_t k = take ? (deg + kSpan - 1) / kSpan : 0u;
@@ -86,7 +87,9 @@ __device__ __forceinline__ void append_entries(uint2* list, uint32_t* count, boo
   }
   uint32_t base = 0;
   if (lane == 31) base = atomicAdd(count, incl);
-  base = __shfl_sync(FULL, base, 31) + incl - k;
+  base = __shfl_sync(FULL, base, 31);
+  if (base + __shfl_sync(FULL, incl, 31) >= limit) return;
+  base += incl - k;
   if (k && k <= 32)
     for (uint32_t i = 0; i < k; i++) list[base + i] = make_uint2(v, i * kSpan);
   for (uint32_t big = __ballot_sync(FULL, k > 32); big; big &= big - 1) {  // a hub: the warp's lanes together
