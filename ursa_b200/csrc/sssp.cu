@@ -35,6 +35,7 @@ constexpr double kDeltaWeights = 1.0;
 constexpr uint64_t kPlainEdges = 1u << 20;
 constexpr uint64_t kStepEntries = 32768;  // a step of fewer entries is small;
 constexpr unsigned kSmallSteps = 4;       // past this many in a row every further one is doubled
+constexpr double kGapSteps = 8.0;         // a gap of more is jumped (jumping any: log-normal weights 8.2 -> 8.5 ms)
 constexpr int kSsspBlocks = 8;         // per SM
 
 __device__ __forceinline__ void append_w(uint32_t* Q, uint32_t* cnt, bool take, uint32_t v) {
@@ -58,8 +59,9 @@ __device__ __forceinline__ unsigned long long ld_bits(const unsigned long long* 
 // per run of them.  Near rounds relax the out-edges of the near list (entries
 // of 16 edges); a node whose distance falls below the threshold joins the
 // next near list (once per round: `stamp`), others the far list (once: `far`).
-// With nothing near, the threshold moves up by delta and a refill round moves
-// the far nodes below it to the near list (the near-far form of
+// With nothing near, the threshold moves up by delta (or, past a wide gap, to the
+// nearest far node and delta) and a refill round moves the far nodes below it
+// to the near list (the near-far form of
 // delta-stepping, Davidson et al.).  Any order reaches the same fixpoint; this
 // one relaxes fewer edges whose source is still to fall.
 enum SsspMode : uint32_t { kNear = 0, kRefill = 1, kSsspDone = 2 };
@@ -73,6 +75,7 @@ struct SsspState {
   double threshold, delta;
   unsigned long long walked;  // entries since the threshold moved
   double reached;  // the threshold before: distances below it have been queued as they fell
+  unsigned long long far_min;  // of a refill: the least distance left far
 };
 
 struct SsspArgs {
@@ -112,6 +115,7 @@ __global__ void __launch_bounds__(1024) sssp_init_k(SsspArgs a, uint32_t source,
   s.mode = entries ? kNear : kSsspDone;
   s.entries[0] = entries;
   s.threshold = s.delta = delta;
+  s.far_min = ~0ull;
   *a.st = s;
 }
 
@@ -164,6 +168,7 @@ __global__ void __launch_bounds__(kBlock) sssp_round_k(SsspArgs a) {
     const uint32_t from = sp->far_buf, count = sp->fars[from];
     const uint32_t* list = a.far_list[from];
     const uint64_t span = (count + nthr - 1) / nthr * nthr;
+    unsigned long long least = ~0ull;
     for (uint64_t i = gtid; i < span; i += nthr) {
       bool near = false, far = false;
       uint32_t v = 0, deg = 0;
@@ -171,6 +176,7 @@ __global__ void __launch_bounds__(kBlock) sssp_round_k(SsspArgs a) {
         v = list[i];
         const unsigned long long d = a.dist[v];
         far = d >= below;
+        if (far) least = min(least, d);
         near = !far && d >= done;
         if (!far) a.far[v] = 0u;
       }
@@ -178,6 +184,9 @@ __global__ void __launch_bounds__(kBlock) sssp_round_k(SsspArgs a) {
       append_entries(a.list[parity], &a.st->entries[parity], near, v, deg);
       append_w(a.far_list[from ^ 1], &a.st->fars[from ^ 1], far, v);
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) least = min(least, __shfl_xor_sync(FULL, least, o));
+    if ((threadIdx.x & 31) == 0 && least != ~0ull) atomicMin(&a.st->far_min, least);
   }
   __syncthreads();
   if (threadIdx.x) return;
@@ -200,7 +209,14 @@ __global__ void __launch_bounds__(kBlock) sssp_round_k(SsspArgs a) {
     s->small_steps = s->walked < kStepEntries ? s->small_steps + 1 : 0;
     if (s->small_steps > kSmallSteps) s->delta *= 2.0;
     s->walked = 0;
-    const double t = s->threshold + s->delta;
+    double t = s->threshold + s->delta;
+    // a refill that found nothing near has seen every far node: past a wide
+    // gap, on to the nearest (one weight in a thousand 1, the others 1e-12, a
+    // million nodes: 2.9 ms a call in steps of delta, 2.5 so)
+    if (mode == kRefill) {
+      const double nearest = __longlong_as_double((long long)__ldcg(&s->far_min));
+      if (nearest - s->threshold > kGapSteps * s->delta) t = nearest + s->delta;
+    }
     s->reached = s->threshold;
     if (t > s->threshold) {
       s->threshold = t;
@@ -209,6 +225,7 @@ __global__ void __launch_bounds__(kBlock) sssp_round_k(SsspArgs a) {
       s->threshold = s->delta;
     }
   }
+  s->far_min = ~0ull;
   s->mode = near ? kNear : fars ? kRefill : kSsspDone;
   s->entries[round & 1] = 0;
   s->round = round + 1;
