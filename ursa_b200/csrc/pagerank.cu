@@ -1553,7 +1553,7 @@ void pagerank_run(TopoImpl* t, const ursa_gpu_pagerank_params& p, const double* 
   if (stats) *stats = ursa_gpu_pagerank_stats{0, 0.0, 0.0};
   if (n == 0) return;
   const bool weighted = d_weights != nullptr;
-  if (!weighted && pagerank_small_fits(t)) {
+  if (!weighted && pagerank_small_fits(t, s)) {
     pagerank_small_run(t, p, d_out, s, stats);
     return;
   }

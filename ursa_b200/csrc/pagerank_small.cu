@@ -4,21 +4,23 @@
 // On a graph of a thousand nodes the persistent kernel of pagerank.cu spends
 // its time on what makes it fast on a large one: per iteration every block
 // loads a 192 KB slice of shares and crosses two grid barriers (about 17 us),
-// after an execution layout that costs a new topology 0.4 ms and more.  Here one cluster of eight CTAs runs the
-// whole call straight from the in-CSR: each CTA owns a run of rows (equal
-// rows + edges), keeps every node's share in its own shared memory, and
-// writes a row's new share to all eight (distributed shared memory), so an
-// iteration costs one cluster barrier and no trip to L2 for the shares.  The
-// row's sources are kept in shared memory too, as 16-bit ids, when they fit.
+// after an execution layout that costs a new topology 0.4 ms and more.  Here
+// one cluster of eight CTAs runs the whole call straight from the in-CSR: each
+// CTA owns a run of rows (equal rows + edges), keeps every node's share in its
+// own shared memory, and writes a row's new share to all eight (distributed
+// shared memory), so an iteration costs one cluster barrier and no trip to L2
+// for the shares.  The rows' sources are kept in shared memory too, as 16-bit
+// ids: those of long rows always, the others where they fit.
 // The arithmetic is pagerank.cu's, operation for operation: f32 shares, a row
 // of up to 64 in-edges summed by one lane in CSR order with a compensated f32
 // pair, longer rows in pieces of 128 edges combined in that kernel's order;
 // f64 ranks; residual and dangling mass summed exactly, in fixed point.  So
 // both kernels give the same ranks bit for bit on the graphs compared.  A call
-// on 1,000 nodes, 10,000 edges: 234 us before, 73 now (70 with f64 sums, which
-// depend on their order); R-MAT with 14,336 nodes and 140,000 edges: 287 and
-// 200.  What is left is the launch and, per iteration, the chain of one row's
-// additions, two block-wide waits and the cluster barrier (about 4 us).
+// on 1,000 nodes, 10,000 edges: 234 us before, 70 now; 30 iterations on R-MAT
+// with 14,336 nodes and 140,000 edges, ranks to the host: 591 and 475; with
+// 2,000 nodes and 200,000 edges 642 and 397.  What is left is the launch and,
+// per iteration, the chain of one row's additions, the block-wide waits and the
+// cluster barrier (about 4 us).
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -36,19 +38,21 @@ namespace {
 constexpr int kCtas = 8;  // the portable cluster size
 constexpr int kThreads = 1024;
 constexpr int kWarps = kThreads / 32;
-// A CTA holds two share buffers (8 bytes a node), at most a quarter of the
-// rows and one (18 bytes a row), and the pieces of its long rows (12 bytes
-// each): at most one per 64 edges of an eighth of rows * row_cost + edges,
-// and those of the row that crosses its end.
+// What a CTA keeps in shared memory has to fit (small_bytes): two share
+// buffers (8 bytes a node), its rows (18 bytes each, at most a quarter of all
+// and one), and its rows of more than 64 edges with their pieces and sources.
+// Those are the larger part of a skewed graph's edges, and a lane walks one
+// piece: from global memory every lane would read a line of its own, so a graph
+// whose pieces do not fit takes the large kernel.  (One hub of 100,000 edges:
+// 2,170 us a call with its sources in global memory, 635 with the large kernel.)
 constexpr uint64_t kMaxNodes = 14336;
-constexpr uint64_t kMaxEdges = 1u << 18;  // R-MAT with 14,336 nodes: 224,000 edges 236 us (275), twice that slower
-constexpr uint64_t kMaxPieces = (2 * kMaxEdges + kMaxNodes) / 8 / 64 + kMaxEdges / 128 + 2;
+constexpr uint64_t kMaxEdges = 1u << 18;  // more: the large kernel is as fast
 constexpr size_t kSmemBytes = 227u * 1024u - 3u * 1024u;  // under 2 KB are static
 static_assert(kWarps == 32, "one warp sums the warps' sums");
-static_assert(8 * kMaxNodes + 18 * (kMaxNodes / 4 + 2) + 12 * kMaxPieces + 32 <= kSmemBytes, "a CTA's rows fit");
 constexpr uint32_t kShort = 8;     // rows up to this are kept together, so that lanes end together
 constexpr uint32_t kDirect = 64;   // rows up to this: one lane
 constexpr uint32_t kPiece = 128;   // longer ones: a lane per piece of this many edges,
+constexpr uint32_t kPieceStride = kPiece + 2;  // u16 between two pieces' sources: an odd number of banks
 constexpr uint32_t kWide = 32;     // combined by one lane up to this many pieces, else a warp
 
 struct SmallArgs {
@@ -83,8 +87,8 @@ struct Sums {
 };
 
 // Sums over the warp, valid in every lane: limbs of 26 bits, whose 32-lane
-// sums fit the 32 bits of a warp-wide add (shuffles of whole words: 90 us
-// against 73 for a call on 1,000 nodes).
+// sums fit the 32 bits of a warp-wide add (shuffles of whole words: 20 us
+// more for a call on 1,000 nodes).
 __device__ __forceinline__ u128 warp_sum(u128 v) {
   constexpr int kBits = 26;
   if (!__any_sync(0xffffffffu, v != 0)) return 0;  // warps without rows, graphs without dangling nodes
@@ -191,8 +195,8 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1) pr_
     }
     ends[k] = filled;
   }
-  // pieces of the long rows, in row order: first piece of each (one past the
-  // last closes the list), and each piece's place in the list
+  // the long rows: edges before each (those of long rows alone), first edge,
+  // first piece (one past the last closes both lists); and each piece's row
   const uint32_t n_long = ends[2] - ends[1];
   const uint16_t* longs = by_len + ends[1];
   const size_t used = reinterpret_cast<unsigned char*>(by_len + rows) - smem;
@@ -205,31 +209,70 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1) pr_
   }
   __syncthreads();
   const uint32_t n_pieces = s_warp[0];
-  uint16_t* piece_row = reinterpret_cast<uint16_t*>(partial + n_pieces);
+  uint32_t* before = reinterpret_cast<uint32_t*>(partial + n_pieces);
+  uint32_t* begin = before + n_long + 1;
+  uint16_t* piece_row = reinterpret_cast<uint16_t*>(begin + n_long);
   uint16_t* first_piece = piece_row + n_pieces;
   if (threadIdx.x < 32) {
-    uint32_t at = 0;
+    uint32_t at = 0, ate = 0;
     for (uint32_t ib = 0; ib < n_long; ib += 32) {
       const uint32_t i = ib + lane;
-      const uint32_t c = i < n_long ? (off[longs[i] + 1] - off[longs[i]] + kPiece - 1) / kPiece : 0u;
-      uint32_t incl = c;
+      const uint32_t b = i < n_long ? off[longs[i]] : 0u;
+      const uint32_t len = i < n_long ? off[longs[i] + 1] - b : 0u;
+      const uint32_t c = (len + kPiece - 1) / kPiece;
+      uint32_t incl = c, incle = len;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
+        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o), te = __shfl_up_sync(0xffffffffu, incle, o);
+        if (lane >= o) {
+          incl += t;
+          incle += te;
+        }
       }
-      if (i < n_long) first_piece[i] = (uint16_t)(at + incl - c);
+      if (i < n_long) {
+        first_piece[i] = (uint16_t)(at + incl - c);
+        before[i] = ate + incle - len;
+        begin[i] = b;
+      }
       at += __shfl_sync(0xffffffffu, incl, 31);
+      ate += __shfl_sync(0xffffffffu, incle, 31);
     }
-    if (lane == 0) first_piece[n_long] = (uint16_t)at;
+    if (lane == 0) {
+      first_piece[n_long] = (uint16_t)at;
+      before[n_long] = ate;
+    }
   }
   __syncthreads();
   for (uint32_t i = threadIdx.x; i < n_long; i += kThreads)
     for (uint32_t q = first_piece[i]; q < first_piece[i + 1]; q++) piece_row[q] = (uint16_t)i;
-  uint16_t* src = first_piece + n_long + 1;
-  const bool cached = reinterpret_cast<unsigned char*>(src + edges) <= smem + kSmemBytes;
-  if (cached)
+  // from here on off[] counts the edges of the other rows alone
+  if (n_long)
+    for (uint32_t r = threadIdx.x; r <= rows; r += kThreads) {
+      uint32_t lo = 0, hi = n_long;  // long rows before r
+      while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (longs[mid] < r) lo = mid + 1; else hi = mid;
+      }
+      off[r] -= before[lo];
+    }
+  __syncthreads();
+  auto piece_end = [&](uint32_t i, uint32_t b) { return min(b + kPiece, begin[i] + before[i + 1] - before[i]); };
+  // sources: of the pieces first, kPieceStride apart, then of the other rows
+  uint16_t* psrc = first_piece + n_long + 1;
+  const bool pcached = reinterpret_cast<unsigned char*>(psrc + n_pieces * kPieceStride) <= smem + kSmemBytes;
+  uint16_t* src = psrc + (pcached ? n_pieces * kPieceStride : 0u);
+  const bool cached = reinterpret_cast<unsigned char*>(src + off[rows]) <= smem + kSmemBytes;
+  if (pcached)
+    for (uint32_t q = threadIdx.x >> 5; q < n_pieces; q += kWarps) {
+      const uint32_t i = piece_row[q], b = begin[i] + (q - first_piece[i]) * kPiece, e = piece_end(i, b);
+      for (uint32_t k = b + lane; k < e; k += 32) psrc[q * kPieceStride + k - b] = (uint16_t)a.in_src[e0 + k];
+    }
+  if (cached && !n_long)
     for (uint32_t k = threadIdx.x; k < edges; k += kThreads) src[k] = (uint16_t)a.in_src[e0 + k];
+  else if (cached)
+    for (uint32_t r = threadIdx.x; r < rows; r += kThreads)
+      for (uint32_t b = off[r], k = 0, g = a.in_off[r0 + r]; k < off[r + 1] - b; k++)
+        src[b + k] = (uint16_t)a.in_src[g + k];
   cluster.sync();
   uint32_t it = 0;
   double2 sums = total(part[0]);
@@ -251,29 +294,25 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1) pr_
 #pragma unroll
       for (int c = 0; c < kCtas; c++) cluster.map_shared_rank(nxt, c)[r0 + r] = share;
     };
-    auto gather = [&](uint32_t k) { return cur[cached ? (uint32_t)src[k] : a.in_src[e0 + k]]; };
-    auto sum = [&](uint32_t b, uint32_t e) {  // Kahan, in CSR order
+    auto sum = [&](const uint16_t* kept, const uint32_t* far, uint32_t len) {  // Kahan, in CSR order
       float v = 0.f, c = 0.f;
-      for (uint32_t k = b; k < e; k++) {
-        const float y = __fsub_rn(gather(k), c);
+      for (uint32_t k = 0; k < len; k++) {
+        const float y = __fsub_rn(cur[kept ? (uint32_t)kept[k] : far[k]], c);
         const float t = __fadd_rn(v, y);
         c = __fsub_rn(__fsub_rn(t, v), y);
         v = t;
       }
       return F2{v, -c};
     };
-    for (uint32_t i = threadIdx.x; i < ends[0]; i += kThreads) {
-      const uint32_t r = by_len[i];
-      finish(r, f2_value(sum(off[r], off[r + 1])));
-    }
-    for (uint32_t i = ends[0] + threadIdx.x; i < ends[1]; i += kThreads) {
-      const uint32_t r = by_len[i];
-      finish(r, f2_value(sum(off[r], off[r + 1])));
-    }
+    auto row_sum = [&](uint32_t r) {
+      return f2_value(sum(cached ? src + off[r] : nullptr, cached ? nullptr : a.in_src + a.in_off[r0 + r],
+                          off[r + 1] - off[r]));
+    };
+    for (uint32_t i = threadIdx.x; i < ends[0]; i += kThreads) finish(by_len[i], row_sum(by_len[i]));
+    for (uint32_t i = ends[0] + threadIdx.x; i < ends[1]; i += kThreads) finish(by_len[i], row_sum(by_len[i]));
     for (uint32_t q = threadIdx.x; q < n_pieces; q += kThreads) {
-      const uint32_t i = piece_row[q], r = longs[i];
-      const uint32_t b = off[r] + (q - first_piece[i]) * kPiece;
-      partial[q] = sum(b, min(b + kPiece, off[r + 1]));
+      const uint32_t i = piece_row[q], b = begin[i] + (q - first_piece[i]) * kPiece;
+      partial[q] = sum(pcached ? psrc + q * kPieceStride : nullptr, a.in_src + e0 + b, piece_end(i, b) - b);
     }
     if (n_long) {
       __syncthreads();
@@ -322,7 +361,62 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1) pr_
 
 }  // namespace
 
-bool pagerank_small_fits(const TopoImpl* t) { return t->n <= kMaxNodes && t->m <= kMaxEdges; }
+// Shared memory of a CTA up to its pieces' sources.
+static __host__ __device__ uint64_t small_bytes(uint64_t n, uint64_t rows, uint64_t longs, uint64_t pieces) {
+  return (8 * n + 18 * rows + 4 + 7) / 8 * 8 + 10 * pieces + 10 * (longs + 1) + 2 * kPieceStride * pieces;
+}
+
+// Whether every CTA's rows and pieces fit.
+__global__ void __launch_bounds__(kThreads) pr_small_check_k(SmallArgs a, uint32_t* fits) {
+  __shared__ uint32_t s_rows[kCtas + 1], pieces[kCtas], longs[kCtas];
+  if (threadIdx.x <= kCtas) s_rows[threadIdx.x] = threadIdx.x == kCtas ? a.n : first_row(a, threadIdx.x);
+  if (threadIdx.x < kCtas) pieces[threadIdx.x] = longs[threadIdx.x] = 0;
+  __syncthreads();
+  for (uint32_t r = threadIdx.x; r < a.n; r += kThreads) {
+    const uint32_t len = a.in_off[r + 1] - a.in_off[r];
+    if (len <= kDirect) continue;
+    uint32_t c = 0;
+    while (r >= s_rows[c + 1]) c++;
+    atomicAdd(&pieces[c], (len + kPiece - 1) / kPiece);
+    atomicAdd(&longs[c], 1u);
+  }
+  __syncthreads();
+  if (threadIdx.x) return;
+  bool all = true;
+  for (int c = 0; c < kCtas; c++)
+    all = all && small_bytes(a.n, s_rows[c + 1] - s_rows[c], longs[c], pieces[c]) <= kSmemBytes;
+  *fits = all;
+}
+
+static SmallArgs small_args(TopoImpl* t) {
+  SmallArgs a{};
+  a.in_off = t->in.off.get();
+  a.in_src = t->in.tgt.get();
+  a.out_off = t->out.off.get();
+  a.n = (uint32_t)t->n;
+  a.m = (uint32_t)t->m;
+  a.row_cost = (uint32_t)std::max<uint64_t>(1, (t->m + t->n - 1) / t->n);
+  return a;
+}
+
+// Looked at once per topology, and not where any graph of its size fits.
+bool pagerank_small_fits(TopoImpl* t, cudaStream_t s) {
+  if (t->n > kMaxNodes || t->m > kMaxEdges) return false;
+  const uint64_t longs = t->m / (kDirect + 1), pieces = longs + t->m / kPiece;  // at most
+  if (small_bytes(t->n, t->n / 4 + 2, longs, pieces) <= kSmemBytes) return true;
+  ensure_in(t, s);
+  std::lock_guard<std::mutex> g(t->mu);
+  if (t->pr_small < 0) {
+    Scratch<uint32_t> fits(1, s);
+    pr_small_check_k<<<1, kThreads, 0, s>>>(small_args(t), fits.get());
+    UG_LAUNCH_CHECK();
+    uint32_t f = 0;
+    UG_CUDA(cudaMemcpyAsync(&f, fits.get(), sizeof(f), cudaMemcpyDeviceToHost, s));
+    UG_CUDA(cudaStreamSynchronize(s));
+    t->pr_small = (int)f;
+  }
+  return t->pr_small != 0;
+}
 
 void pagerank_small_run(TopoImpl* t, const ursa_gpu_pagerank_params& p, double* d_out, cudaStream_t s,
                         ursa_gpu_pagerank_stats* stats) {
@@ -337,19 +431,11 @@ void pagerank_small_run(TopoImpl* t, const ursa_gpu_pagerank_params& p, double* 
       ready[t->device] = true;
     }
   }
-  SmallArgs a;
-  a.in_off = t->in.off.get();
-  a.in_src = t->in.tgt.get();
-  a.out_off = t->out.off.get();
-  a.n = (uint32_t)t->n;
-  a.m = (uint32_t)t->m;
+  SmallArgs a = small_args(t);
   a.damping = p.damping;
   a.tol = p.tol;
   a.max_iter = p.max_iter;
-  a.row_cost = (uint32_t)std::max<uint64_t>(1, (t->m + t->n - 1) / t->n);
   a.out = d_out;
-  a.delta_out = nullptr;
-  a.iters_out = nullptr;
   Scratch<double> info;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (stats) {

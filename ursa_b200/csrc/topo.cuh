@@ -44,6 +44,7 @@ struct TopoImpl {
     uint64_t n_hubs = 0, n_chunks = 0;
     bool built = false;
   } ms_hubs[3];
+  int pr_small = -1;  // 0/1: whether one cluster takes PageRank, -1: not looked at (pagerank_small.cu)
   PrPlan* pr_plan = nullptr;
   // a plan without edge ids, replaced by one with them for a weighted call;
   // kept until the topology goes (a call on another thread may still use it)
@@ -89,7 +90,7 @@ void pagerank_run(TopoImpl* t, const ursa_gpu_pagerank_params& p, const double* 
                   double* d_out, cudaStream_t s, ursa_gpu_pagerank_stats* stats);
 // The same for graphs that fit one thread-block cluster, unweighted
 // (pagerank_small.cu).
-bool pagerank_small_fits(const TopoImpl* t);
+bool pagerank_small_fits(TopoImpl* t, cudaStream_t s);
 void pagerank_small_run(TopoImpl* t, const ursa_gpu_pagerank_params& p, double* d_out, cudaStream_t s,
                         ursa_gpu_pagerank_stats* stats);
 void cc_weak_run(TopoImpl* t, uint32_t* d_out, cudaStream_t s);
