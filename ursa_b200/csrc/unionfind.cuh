@@ -17,9 +17,10 @@ __device__ __forceinline__ uint32_t uf_parent(const uint32_t* p, uint32_t x) {
 }
 
 // The same read through L1 (global memory only).  A cached parent may be
-// stale, which costs steps and no correctness: what was once an ancestor of x
-// stays one, parents stay smaller than their children, and a stale root is
-// found out by the compare-and-swap that hooks it.  Reads past L1 all meet at
+// stale, which costs steps and no correctness: a jump may have taken it off
+// x's path, but two nodes once in one set stay in one, parents stay smaller
+// than their children, and a stale root is found out by the compare-and-swap
+// that hooks it.  Reads past L1 all meet at
 // the L2 slice that holds the largest tree's root.
 __device__ __forceinline__ uint32_t uf_parent_l1(const uint32_t* p, uint32_t x) {
   uint32_t v;
@@ -44,10 +45,15 @@ __device__ __forceinline__ uint32_t uf_find(uint32_t* p, uint32_t x) {
 // The same through L1.  Short walks store x's parent alone: the nodes further
 // up are those that every walk passes, and their stores would meet at a few
 // addresses.  Past kUfShort links a walk reads past L1, wanting the jumps that
-// others have stored, and stores its own.  (Jumps from the first link on:
-// R-MAT-16's components 153 us a call, 115 so; a path of a million nodes in
-// random order 1,105 and 742.)
-constexpr int kUfShort = 4;
+// others have stored, and stores its own.  Four links are too few where trees
+// are a dozen deep: the last ones, near a root that all walks share, then meet
+// at its L2 slice.  Kernels of a call with 4 / 8 / 16 / 32 (and before, with
+// jumps from the first link on, past L1), us: four million nodes with twice as
+// many random edges 1,864 / 828 / 765 / 939 (922), with 1.5 times 718 / 519 /
+// 615 / 797 (524), three times 934 / 675 / 688 / 902 (793); a path of four
+// million nodes in random order 889 / 511 / 426 / 424 (1,212); R-MAT with four
+// million nodes 384 / 398 / 405 / 396 (1,933).
+constexpr int kUfShort = 8;
 __device__ __forceinline__ uint32_t uf_find_l1(uint32_t* p, uint32_t x) {
   uint32_t par = uf_parent_l1(p, x);
   if (par != x) {
