@@ -236,6 +236,7 @@ __global__ void cc_rest_k(const uint32_t* __restrict__ off, const uint32_t* __re
 // Every out-edge that the giant does not hold on both ends, one thread per
 // slot: only when no root owns half of the edges, or a row outside the giant
 // is too long for a warp (balanced whatever the degrees).
+template <bool kL1>
 __global__ void cc_slots_k(const uint32_t* __restrict__ off, const uint32_t* __restrict__ tgt,
                            uint64_t n, uint64_t m, uint32_t* parent, const CcCtl* ctl) {
   if (ctl && !ctl->by_slot) return;
@@ -244,7 +245,7 @@ __global__ void cc_slots_k(const uint32_t* __restrict__ off, const uint32_t* __r
     const uint32_t v = tgt[k];
     if (u == v) return;
     if (giant != kNoGiant && uf_parent(parent, u) == giant && uf_parent(parent, v) == giant) return;
-    uf_unite<true>(parent, u, v);
+    uf_unite<kL1>(parent, u, v);
   });
 }
 
@@ -282,7 +283,9 @@ void cc_weak_with_parent(TopoImpl* t, uint32_t* parent, uint32_t* d_out, cudaStr
     iota_k<<<grid_for(n), kBlock, 0, s>>>(parent, n);
     UG_LAUNCH_CHECK();
     if (m) {
-      cc_slots_k<<<grid_for(m, kBlock, 148u * 64u), kBlock, 0, s>>>(off, tgt, n, m, parent, nullptr);
+      // finds past L1 where trees stay small (four million nodes, two million edges: 155 us, 163 through L1)
+      auto slots = m < kSampleEdges ? cc_slots_k<true> : cc_slots_k<false>;
+      slots<<<grid_for(m, kBlock, 148u * 64u), kBlock, 0, s>>>(off, tgt, n, m, parent, nullptr);
       UG_LAUNCH_CHECK();
     }
   } else {
@@ -296,7 +299,7 @@ void cc_weak_with_parent(TopoImpl* t, uint32_t* parent, uint32_t* d_out, cudaStr
     UG_LAUNCH_CHECK();
     cc_rest_k<<<grid_for(n), kBlock, 0, s>>>(off, tgt, in_off, in_tgt, n, parent, ctl);
     UG_LAUNCH_CHECK();
-    cc_slots_k<<<grid_for(m, kBlock, 148u * 64u), kBlock, 0, s>>>(off, tgt, n, m, parent, ctl);
+    cc_slots_k<true><<<grid_for(m, kBlock, 148u * 64u), kBlock, 0, s>>>(off, tgt, n, m, parent, ctl);
     UG_LAUNCH_CHECK();
   }
   flatten_k<<<grid_for(n, kBlock, kRuns), kBlock, 0, s>>>(parent, n, d_out);
