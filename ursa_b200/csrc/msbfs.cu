@@ -475,15 +475,22 @@ __global__ void __launch_bounds__(kMsBlock, W == 4 ? kMsOcc : kMsOcc1) ms_persis
 
 static_assert(kMsBlockNodes == 32 * kMsWarps, "a warp per 32 nodes");
 
-// Blocks of either variant (with and without groups) that are resident at once.
+// Blocks of either variant (with and without groups) that are resident at
+// once; asked once per device.
 template <int W>
 uint64_t ms_resident(int device) {
-  int a = 0, b = 0;
-  UG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, ms_persist_k<W, true>, kMsBlock, 0));
-  UG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, ms_persist_k<W, false>, kMsBlock, 0));
-  const int per_sm = std::min(a, b);
-  UG_CHECK(per_sm > 0, URSA_GPU_ECUDA, "msbfs: kernel cannot be resident");
-  return (uint64_t)per_sm * sm_count(device);
+  static std::mutex mu;
+  static int per_sm[64] = {0};
+  UG_CHECK(device >= 0 && device < 64, URSA_GPU_EINVAL, "device index out of range");
+  std::lock_guard<std::mutex> g(mu);
+  if (!per_sm[device]) {
+    int a = 0, b = 0;
+    UG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, ms_persist_k<W, true>, kMsBlock, 0));
+    UG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, ms_persist_k<W, false>, kMsBlock, 0));
+    UG_CHECK(std::min(a, b) > 0, URSA_GPU_ECUDA, "msbfs: kernel cannot be resident");
+    per_sm[device] = std::min(a, b);
+  }
+  return (uint64_t)per_sm[device] * sm_count(device);
 }
 
 template <int W>
@@ -766,10 +773,10 @@ static void msbfs_enqueue(TopoImpl* t, int dir, const uint32_t* d_src, uint64_t 
   a.group_blocks = shape.group_blocks;
   const uint64_t words = a.groups * n * W;
   Scratch<unsigned long long> visited(words, s), fa(words, s), fb(words, s), acc(words, s);
-  Scratch<unsigned long long> count(a.groups * 3 * (64 * W + 8), s);
-  Scratch<unsigned> bar(a.groups * 2, s);
+  // a word per group's barrier (count, generation), then its counters
+  Scratch<unsigned long long> count(a.groups * (1 + 3 * (64 * W + 8)), s);
   UG_CUDA(cudaMemsetAsync(acc.get(), 0, words * 8, s));
-  UG_CUDA(cudaMemsetAsync(bar.get(), 0, a.groups * 2 * sizeof(unsigned), s));
+  UG_CUDA(cudaMemsetAsync(count.get(), 0, a.groups * sizeof(unsigned long long), s));
   const uint64_t nh = hb.n_hubs, nc = hb.n_chunks;
   const uint64_t hub_words = a.groups * (nh ? nh : 1) * W;
   Scratch<unsigned long long> hacc(hub_words, s);
@@ -794,11 +801,11 @@ static void msbfs_enqueue(TopoImpl* t, int dir, const uint32_t* d_src, uint64_t 
   a.chunk_lo = hb.chunk_lo.get();
   a.n_chunks = nc;
   a.hacc = hacc.get();
-  a.count = count.get();
+  a.count = count.get() + a.groups;
   a.reach = d_reach;
   a.dsum = d_dsum;
   a.maxd = d_maxd;
-  a.bar = bar.get();
+  a.bar = reinterpret_cast<unsigned*>(count.get());
   a.err = (int*)(d_ctl + 2);
   if (W == 4)
     ms_launch<4>(a, n_sources, s);
