@@ -244,7 +244,7 @@ int ursa_gpu_clustering_coefficient(ursa_gpu_topo *t, double *out);
 /* betweenness(&Topology, Option<f64>, Option<u64>) -> Vec<f64> --
  * algo/betweenness.rs:153-177.  has_sample/has_seed encode the Options.  The
  * sampled source set is the reference's seeded shuffled_order prefix
- * (betweenness.rs:349-362, rng.rs:64-72), computed on the host. */
+ * (betweenness.rs:349-362, rng.rs:64-72). */
 int ursa_gpu_betweenness(ursa_gpu_topo *t, int has_sample, double sample, int has_seed,
                          uint64_t seed, double *out);
 /* betweenness_weighted(&Topology, &[f64], Option<f64>, Option<u64>) --

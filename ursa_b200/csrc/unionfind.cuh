@@ -4,8 +4,11 @@
 //
 // A union always hooks the larger root under the smaller one with a
 // compare-and-swap (a failed CAS means the root moved; the walk continues from
-// the new parent), and finds compress paths by pointer jumping.  Parents only
-// ever decrease, so each tree's root is the minimum id of its component.
+// the new parent), and finds compress paths by pointer jumping: the find with
+// intermediate pointer jumping and the hooking of ECL-CC (Jaiganesh and
+// Burtscher, "A High-Performance Connected Components Implementation for
+// GPUs").  Parents only ever decrease, so each tree's root is the minimum id of
+// its component.
 #pragma once
 
 #include <stdint.h>
