@@ -380,7 +380,7 @@ __device__ void bk_components(BkShared& sh, uint32_t* par) {
 // found in the bitmap closes the triangle {u, v, w}, counted once (u < v < w
 // in the orientation's rank order) and credited to all three vertices: u's
 // and v's credit once per list (the counts of tc_stream), w's per hit.  Graphs
-// above kTcBitCap nodes use a per-lane sorted merge.  Bound by issue (0.58 of a
+// above kTcBitCap nodes use a per-lane sorted merge.  Bound by issue (0.66 of a
 // slot per scheduler and cycle, 65 instructions per 32 probes) and by how
 // unevenly the units weigh: 1,000 graphs 9.65 ms before the shared probe loop
 // with the next elements in flight, 8.0 now; units of 8 or 16 vertices pay

@@ -6,8 +6,8 @@
 // block to finish decides the next level's way, so levels are enqueued
 // several at a time and the host reads one word per run of them: with a
 // prefix scan of the frontier's degrees and a host read per level, three
-// quarters of a call on 50,000 nodes was launches and round trips (270 us for
-// 70 us of kernels; 99 us now).  R-MAT-22 takes 575 us against 815, 305 of
+// quarters of a call on 50,000 nodes was launches and round trips (297 us for
+// 70 us of kernels; 101 us now).  R-MAT-22 takes 619 us against 875, 305 of
 // them the distances' copy to the host; its pull levels read every unvisited
 // node's row up to its first parent and are bound by those random reads.
 //

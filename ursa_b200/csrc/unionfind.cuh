@@ -55,7 +55,9 @@ __device__ __forceinline__ uint32_t uf_find(uint32_t* p, uint32_t x) {
 // many random edges 1,864 / 828 / 765 / 939 (922), with 1.5 times 718 / 519 /
 // 615 / 797 (524), three times 934 / 675 / 688 / 902 (793); a path of four
 // million nodes in random order 889 / 511 / 426 / 424 (1,212); R-MAT with four
-// million nodes 384 / 398 / 405 / 396 (1,933).
+// million nodes 384 / 398 / 405 / 396 (1,933).  With 4 / 8: R-MAT with one
+// million nodes 325 / 265 (717); sixteen random edges a node, a million nodes,
+// 297 / 345 (752).
 constexpr int kUfShort = 8;
 __device__ __forceinline__ uint32_t uf_find_l1(uint32_t* p, uint32_t x) {
   uint32_t par = uf_parent_l1(p, x);
