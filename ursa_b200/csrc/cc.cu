@@ -16,7 +16,7 @@
 // then only nodes outside that root's tree walk their edges, along both
 // CSRs -- an edge with an end outside is seen from that end, and one with
 // both ends inside joins nothing.  R-MAT-22's kernels took 1,859 us and take
-// about 380 (270 of them the second link's finds); the rest of a 676 us call is
+// about 380 (270 of them the second link's finds); the rest of a 677 us call is
 // the labels' copy to the host.
 #include "frontier.cuh"
 #include "unionfind.cuh"
